@@ -77,6 +77,11 @@ hml_status launch_simt(const GemmProblem &p, const hml_sgemm_config &c, cudaStre
 // only; an explicitly given configuration runs exactly as given).
 hml_status launch_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s,
                      bool waves = false);
+// The split-BF16 form (BF16X6) of a problem whose A TMA cannot address as it
+// stands: an unaligned base or leading dimension (sgemm_tc.cu).  Reached
+// through automatic selection only; explicit configurations refuse such an A.
+bool tc_unaligned_ok(const GemmProblem &p);
+hml_status launch_tc_unaligned(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s);
 hml_status check_simt(const GemmProblem &p, const hml_sgemm_config &c);
 // The stream-K SIMT kernel for N <= 8 with contiguous columns of A
 // (sgemm_stream.cu); reached through the SIMT family's variants

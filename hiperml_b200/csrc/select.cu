@@ -171,4 +171,27 @@ hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t
   return HML_STATUS_SUCCESS;
 }
 
+// Where the tensor cores take a problem whose A TMA cannot address as it
+// stands: wherever they would take it with an addressable A, and from
+// M K max(N, 8) = 2^25 on also where SIMT would.  The SIMT tiles then stage A
+// with 4-byte cp.async and fall behind early (B200, odd K row-major: 2048 x
+// 16 x 1025, at the line, 16.9 us against 16.4; 8192 x 4 x 1025 26.6 against
+// 25.2; 32768 x 8 x 1025 82 against 48; 32768 x 64 x 3001 737 against 119);
+// below it one launch beats two (2048 x 8 x 257 13.2 us against 16.5).
+bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s) {
+  const int64_t ld = p.a_kcontig() ? p.sam : p.sak;
+  const bool base_ok = (reinterpret_cast<uintptr_t>(p.A) & 15u) == 0;
+  if ((base_ok && ld % 4 == 0) || !tc_unaligned_ok(p)) return false;
+  // the choice for the same problem with an addressable A
+  GemmProblem q = p;
+  q.A = reinterpret_cast<const float *>(reinterpret_cast<uintptr_t>(p.A) & ~uintptr_t(15));
+  (p.a_kcontig() ? q.sam : q.sak) = (ld + 3) / 4 * 4;
+  if (select_config(q, c, s) != HML_STATUS_SUCCESS) return false;
+  if (c->algo == HML_ALGO_BF16X6) return true;
+  const double work = static_cast<double>(p.M) * p.K * std::max(p.N, 8);
+  if (c->algo == HML_ALGO_SIMT && work < 0x1p25) return false;
+  *c = heuristic_config(q, HML_ALGO_BF16X6);
+  return true;
+}
+
 }  // namespace hml

@@ -47,6 +47,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -74,6 +75,30 @@ struct TcShape {
 };
 constexpr TcShape kTcShapes[] = {{128, 16}, {128, 32}, {128, 64}, {128, 128}};
 constexpr int kNumTcShapes = sizeof(kTcShapes) / sizeof(kTcShapes[0]);
+
+// How A reaches shared memory.  TMA needs 16-byte aligned bases and strides;
+// an A without them (an odd leading dimension, a shifted base) is still read
+// by TMA, through four maps: the strided lines of A (columns of an
+// M-contiguous A, rows of a K-contiguous one) with index = r mod 4 lie 4 *
+// ld * 4 bytes apart, a multiple of 16, and start e_r = 0..3 floats past a
+// 16-byte boundary.  Map r covers class r from that boundary on, its boxes
+// are 4 floats wider than the block, and the converters skip the e_r floats.
+// (Against the 4-byte cp.async SIMT tiles that served these problems before:
+// 20011 x 45 x 1501 row-major, 293 us -> 52 us a call on B200, A at 2.4 TB/s;
+// what bounds it is the aligned form's converter and handshake pace.)
+enum AMode : int {
+  kAM = 0,   // M-contiguous: one 32 (k) x 128 (m) box a block
+  kAK = 1,   // K-contiguous: one 128 (m) x 32 (k) box, 128-byte swizzle
+  kAMU = 2,  // M-contiguous, unaligned: four 8 (k) x 132 (m) boxes
+  kAKU = 3,  // K-contiguous, unaligned: four 32 (m) x 36 (k) boxes
+};
+__host__ __device__ constexpr bool am_kcontig(int am) { return am == kAK || am == kAKU; }
+__host__ __device__ constexpr bool am_unaligned(int am) { return am >= kAMU; }
+// The maps of A (one, or one per class) and the class offsets e_r.
+template <int AM>
+struct AMaps {
+  CUtensorMap m[am_unaligned(AM) ? 4 : 1];
+};
 
 // Warp roles of one CTA:
 //   warp 0       TMA loads of A (FP32 tiles)
@@ -176,6 +201,13 @@ __device__ __forceinline__ void split_plane32(float (&x)[32], uint32_t (&w)[16])
   }
 }
 
+// x = the 32 values of y from E on.
+template <int E>
+__device__ __forceinline__ void shifted32(const float (&y)[36], float (&x)[32]) {
+#pragma unroll
+  for (int k = 0; k < 32; ++k) x[k] = y[k + E];
+}
+
 // ------------------------------------------------------- FP16X3 split
 // FP16 keeps 11 significant bits but only 5 exponent bits, so each FP32 row
 // block of A (and each column of B) is first scaled by a power of two 2^S
@@ -248,6 +280,7 @@ struct TcArgs {
   int kc;          // K extent per split (multiple of kChunkK)
   int sa, so;      // A ring and operand-stage depths
   int n_pad;       // rows of one B plane in the workspace
+  int e[4];        // unaligned A: floats before the data in class r's boxes
   int *err;
   const int *bexp;  // FP16X3: per column of B, the scale exponent S_n of its planes
 };
@@ -361,28 +394,35 @@ struct TcPlan {
   int sa, so;
 };
 
-__host__ __device__ constexpr size_t tc_a_bytes() { return static_cast<size_t>(kBM) * kBK * 4; }
+// Bytes of the A ring's slots, and of what lands in one: 16 KB, 18 KB for the
+// wider boxes of an unaligned A (132 x 8 boxes leave 1.5 KB of it unused).
+__host__ __device__ constexpr size_t tc_a_bytes(int am = kAM) {
+  return am_unaligned(am) ? 4 * 36 * 32 * 4 : static_cast<size_t>(kBM) * kBK * 4;
+}
+__host__ __device__ constexpr int tc_a_tx(int am) {
+  return am == kAMU ? 4 * 132 * 8 * 4 : static_cast<int>(tc_a_bytes(am));
+}
 __host__ __device__ constexpr size_t tc_b_bytes(int bn, int ns) {
   return static_cast<size_t>(tc_geom(ns)) * bn * kBK * 2;
 }
 // FP16X3: the ring of per-row scale exponents the converters hand to the
 // drain warps, one entry per K block in flight (2 x the operand stages).
 __host__ __device__ constexpr int tc_fh_ring(int so) { return 2 * so; }
-size_t tc_plan_bytes(int bn, int ns, const TcPlan &pl) {
+size_t tc_plan_bytes(int bn, int ns, const TcPlan &pl, int am = kAM) {
   const size_t ring = ns == 5 ? static_cast<size_t>(tc_fh_ring(pl.so)) * (8 + kBM * 4) : 0;
-  return 1024 + pl.sa * tc_a_bytes() + pl.so * tc_b_bytes(bn, ns) +
+  return 1024 + pl.sa * tc_a_bytes(am) + pl.so * tc_b_bytes(bn, ns) +
          8 * (2 * pl.sa + 2 * pl.so + 2 * 4 + 1) + 16 + ring + 16;
 }
 
 // The deepest operand-stage ring that fits TMEM and shared memory next to
 // sa A slots; sa must be a multiple of G.
-bool tc_plan(int bn, int ns, int sa, TcPlan *out) {
+bool tc_plan(int bn, int ns, int sa, TcPlan *out, int am = kAM) {
   const int g = tc_groups();
   if (sa < g || sa % g != 0) return false;
   const int mult = tc_stage_mult(tc_issuers(bn, ns));
   for (int so = tc_max_stages(bn, ns); so >= mult; so -= mult) {
     const TcPlan pl = {sa, so};
-    if (tc_plan_bytes(bn, ns, pl) <= 227 * 1024) {
+    if (tc_plan_bytes(bn, ns, pl, am) <= 227 * 1024) {
       *out = pl;
       return true;
     }
@@ -397,10 +437,11 @@ __host__ __device__ constexpr uint32_t tc_tmem_alloc_cols(int bn, int ns, int so
   return tc_pow2_cols(tc_issuers(bn, ns) * bn + so * tc_stage_cols(ns));
 }
 
-template <int BN, int NS, bool AK>
+template <int BN, int NS, int AM>
 __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
-    tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+    tc_kernel(const __grid_constant__ AMaps<AM> tmA, const __grid_constant__ CUtensorMap tmB,
               TcArgs args) {
+  constexpr bool AK = am_kcontig(AM), AU = am_unaligned(AM);
   // NS = 4 is the TF32 form: 2 planes of 32-bit TF32 (hi, lo), the TMEM and
   // shared-memory footprint of 4 BF16 planes
   constexpr bool TF = NS == 4;
@@ -417,7 +458,7 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
   constexpr int NI = tc_issuers(BN, NS);                     // MMA issuers = accumulators
   constexpr int kThreads = tc_warps(BN, NS) * 32;
   constexpr int kConvWarp0 = tc_conv_warp0(BN, NS), kDrainWarp0 = kConvWarp0 + 4 * G;
-  constexpr int A32_BYTES = static_cast<int>(tc_a_bytes());  // FP32 A slot (16 KB)
+  constexpr int A32_BYTES = static_cast<int>(tc_a_bytes(AM));  // FP32 A slot
   constexpr int BPL_BYTES = BN * kBK * (TF ? 4 : 2);         // one B plane tile
   constexpr int BSLOT = PL * BPL_BYTES;                      // one B slot
   constexpr int SC = tc_stage_cols(NS);                      // TMEM columns of an A stage
@@ -490,7 +531,7 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
   if (warp == 0) {
     // -------------------------------------------------------- TMA, A
     if (lane == 0) {
-      prefetch_tmap(&tmA);
+      for (const CUtensorMap &t : tmA.m) prefetch_tmap(&t);
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % SA;
         if (!mbar_wait(&aempty[s], ((kb / SA) & 1) ^ 1, args.err, kDevErrEmptyBarrier)) {
@@ -499,11 +540,23 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         }
         uint8_t *dst = aring + s * A32_BYTES;
         const int k0 = kbeg + kb * kBK;
-        mbar_arrive_expect_tx(&afull[s], A32_BYTES);
-        if (AK)  // 128 rows of 32 floats (128-byte swizzle)
-          tma_load_2d(dst, &tmA, &afull[s], k0, static_cast<int>(m0));
-        else     // 32 rows (k) of 128 floats (m)
-          tma_load_2d(dst, &tmA, &afull[s], static_cast<int>(m0), k0);
+        mbar_arrive_expect_tx(&afull[s], tc_a_tx(AM));
+        if constexpr (AU) {
+          // class r: rows (columns) r, r + 4, ... of the block, from a
+          // 16-byte boundary; k0 and m0 are multiples of 32
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (AK)
+              tma_load_2d(dst + r * (36 * 32 * 4), &tmA.m[r], &afull[s], k0,
+                          static_cast<int>(m0 / 4));
+            else
+              tma_load_2d(dst + r * (132 * 8 * 4), &tmA.m[r], &afull[s], static_cast<int>(m0),
+                          k0 / 4);
+        } else if (AK) {  // 128 rows of 32 floats (128-byte swizzle)
+          tma_load_2d(dst, &tmA.m[0], &afull[s], k0, static_cast<int>(m0));
+        } else {  // 32 rows (k) of 128 floats (m)
+          tma_load_2d(dst, &tmA.m[0], &afull[s], static_cast<int>(m0), k0);
+        }
       }
     }
   } else if (warp == 1) {
@@ -545,6 +598,27 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
           break;
         }
         const int kb1 = min(nkb, (q + 1) * P);
+        // the products of block kb whose plane indices sum to t0 .. t1, the
+        // smallest (largest sum) first; `fresh` zeroes the accumulator
+        auto issue = [&](int kb, int t0, int t1, bool fresh) {
+          const int o = kb % SO;
+          const uint32_t astage = tA + static_cast<uint32_t>(o * SC);
+          const uint64_t b_desc = sw64_desc(smem_u32(bring + o * BSLOT));
+          uint32_t acc = fresh ? 0u : 1u;
+#pragma unroll
+          for (int t = PL - 1; t >= 0; --t) {
+            if (t < t0 || t > t1) continue;
+#pragma unroll
+            for (int kk = 0; kk < kBK / KMMA; ++kk)
+#pragma unroll
+              for (int i = 0; i <= t; ++i) {
+                mma_bf16_ts(dacc, astage + static_cast<uint32_t>(i * PLC + kk * 8),
+                            b_desc + static_cast<uint64_t>(((t - i) * BPL_BYTES + kk * 32) >> 4),
+                            IDESC, acc);
+                acc = 1u;
+              }
+          }
+        };
         for (int kb = q * P; kb < kb1; ++kb) {
           const int o = kb % SO;
           const bool first = kb == q * P;
@@ -554,6 +628,10 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
             break;
           }
           tc_fence_after();
+          if constexpr (AU) {
+            issue(kb, 1, PL - 1, first);
+            continue;
+          }
           const uint32_t astage = tA + static_cast<uint32_t>(o * SC);
           const uint64_t b_desc = TF ? sw128_desc(smem_u32(bring + o * BSLOT))
                                      : sw64_desc(smem_u32(bring + o * BSLOT));
@@ -578,6 +656,17 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
           }
           mma_commit(&opempty[o]);
         }
+        if constexpr (AU) {
+          // the leading products of the whole chunk last: the tensor core
+          // truncates on every accumulation, so only these 4 of a chunk's 24
+          // lose bits of the full sum (error against FP64 at K = 1501:
+          // 1.2e-7, 5.3e-7 in the order above, 1.8e-7 for the SIMT tiles;
+          // the order above releases a stage earlier, 2 % at N = 128)
+          for (int kb = q * P; ok && kb < kb1; ++kb) {
+            issue(kb, 0, 0, false);
+            mma_commit(&opempty[kb % SO]);
+          }
+        }
         if (ok) mma_commit(&accfull[b]);
       }
       if (!ok) *bad_flag = 1;
@@ -589,6 +678,8 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
     const int g = (warp - kConvWarp0) >> 2;
     const int m = tid & (kBM - 1);  // row of the tile == TMEM lane
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    // kAKU: TMEM lane 32 w + l holds row 4 l + w (class w) of the tile
+    [[maybe_unused]] const int e_w = AM == kAKU ? args.e[warp & 3] : 0;
     for (int kb = g; kb < nkb; kb += G) {
       const int s = kb % SA, o = kb % SO;
       bool w = mbar_wait(&afull[s], (kb / SA) & 1, args.err, kDevErrFullBarrier);
@@ -598,7 +689,27 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
       }
       const float *a32 = reinterpret_cast<const float *>(aring + s * A32_BYTES);
       float x[32];
-      if (AK) {
+      if constexpr (AM == kAKU) {
+        // 36 floats of the lane's row (rows 144 bytes apart: 16-byte reads
+        // without bank conflicts), the block's 32 from e_w on
+        const float *row = a32 + (warp & 3) * (36 * 32) + lane * 36;
+        float y[36];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+          const float4 v = *reinterpret_cast<const float4 *>(row + 4 * c);
+          y[4 * c + 0] = v.x; y[4 * c + 1] = v.y; y[4 * c + 2] = v.z; y[4 * c + 3] = v.w;
+        }
+        switch (e_w) {  // uniform over the warp
+          case 0: shifted32<0>(y, x); break;
+          case 1: shifted32<1>(y, x); break;
+          case 2: shifted32<2>(y, x); break;
+          default: shifted32<3>(y, x); break;
+        }
+      } else if constexpr (AM == kAMU) {
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          x[k] = a32[(k & 3) * (132 * 8) + (k >> 2) * 132 + m + args.e[k & 3]];
+      } else if (AK) {
         // row m holds 32 floats in 128 bytes, 128-byte swizzle
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -797,15 +908,39 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
     __syncthreads();
     const bool failed = *bad_flag != 0;
     float *red = reinterpret_cast<float *>(smem);  // [BN][kBM], reuses the A ring
-    const int m = tid & (kBM - 1);
+    const int m = AM == kAKU ? 4 * lane + (warp & 3) : tid & (kBM - 1);  // row of the tile
     const int64_t gm = m0 + m;
     if (failed) {
 #pragma unroll
       for (int i = 0; i < DC; ++i) sums[i] = 0.0f;
     }
-    if (split > 1) {
+    if (split > 1 || AU) {
 #pragma unroll
       for (int i = 0; i < DC; ++i) red[(d * DC + i) * kBM + m] = sums[i];
+      if constexpr (AU) {
+        // an infinite operand (or one that rounds to BF16's infinity) has
+        // NaN in its residual planes: non-finite sums are formed again in
+        // plain FP32, as the SIMT kernels form them, the lanes of the warp
+        // over k
+        bool odd = false;
+#pragma unroll
+        for (int i = 0; i < DC; ++i) odd |= !(fabsf(sums[i]) <= FLT_MAX);
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(0xffffffffu, odd && gm < p.M); todo;
+             todo &= todo - 1) {
+          const int mr = __shfl_sync(0xffffffffu, m, __ffs(todo) - 1);
+          const float *arow = p.A + (m0 + mr) * p.sam;
+          for (int n = n0 + d * DC; n < min(p.N, n0 + (d + 1) * DC); ++n) {
+            if (fabsf(red[(n - n0) * kBM + mr]) <= FLT_MAX) continue;
+            float v = 0.0f;
+            for (int64_t k = kbeg + lane; k < kend; k += 32)
+              v = fmaf(arow[k * p.sak], p.B[k * p.sbk + n * p.sbn], v);
+            v = warp_sum(v);
+            __syncwarp();
+            if (lane == 0) red[(n - n0) * kBM + mr] = v;
+          }
+        }
+      }
     } else if (gm < p.M) {
 #pragma unroll
       for (int i = 0; i < DC; ++i) {
@@ -820,13 +955,16 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
     }
   }
   if (warp < kDrainWarp0) __syncthreads();
-  if (split > 1) {
+  if (split > 1 || AU) {  // an unaligned A's tile always goes through shared memory
     [[maybe_unused]] int tmax_all = 0;
     if constexpr (FH) {
       wait_prior_grid();  // the column scale exponents below
       tmax_all = *tmax_sh;
     }
-    cluster_sync();
+    if (split > 1)
+      cluster_sync();
+    else
+      __syncthreads();
     const float *red = reinterpret_cast<const float *>(smem);
     constexpr int E = kBM * BN;
     const int per = E / split;
@@ -852,7 +990,7 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         }
       }
     }
-    cluster_sync();
+    if (split > 1) cluster_sync();
   }
   tc_fence_before();
   __syncthreads();
@@ -877,21 +1015,37 @@ bool tc_config_fits(int bn, int ns, int stages) {
 namespace {
 
 // Launch of the kernel with the B planes already split into `planes`.
-template <int BN, int NS, bool AK>
+template <int BN, int NS, int AM>
 hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
                             const __nv_bfloat16 *planes, int k_pad, int n_pad, int *err,
                             cudaStream_t s, const int *bexp = nullptr) {
   if (NS == 5 && !bexp) return HML_STATUS_INVALID_VALUE;
-  CUtensorMap ta, tb;
+  AMaps<AM> ta;
+  CUtensorMap tb;
   memset(&ta, 0, sizeof ta);
   memset(&tb, 0, sizeof tb);
-  bool ok;
-  if (AK)
-    ok = tensor_map_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.K, p.M, p.sam * 4, kBK, kBM,
+  TcArgs args = {};
+  bool ok = true;
+  if constexpr (am_unaligned(AM)) {
+    // lines 4 j + r of A (M and K are at least 4): each class from the
+    // 16-byte boundary at or before its first line, whose granule the
+    // line's first float shares
+    const bool ak = AM == kAKU;
+    const int64_t ld = ak ? p.sam : p.sak;
+    const int lines = ak ? p.M : p.K, len = ak ? p.K : p.M;
+    for (int r = 0; r < 4 && ok; ++r) {
+      const float *first = p.A + r * ld;
+      args.e[r] = static_cast<int>((reinterpret_cast<uintptr_t>(first) & 15u) / 4);
+      ok = tensor_map_2d(&ta.m[r], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, first - args.e[r],
+                         len + args.e[r], (lines - r + 3) / 4, ld * 16, ak ? 36 : 132,
+                         ak ? 32 : 8, CU_TENSOR_MAP_SWIZZLE_NONE);
+    }
+  } else if (AM == kAK)
+    ok = tensor_map_2d(&ta.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.K, p.M, p.sam * 4, kBK, kBM,
                        CU_TENSOR_MAP_SWIZZLE_128B);
   else
-    ok = tensor_map_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.M, p.K, p.sak * 4, kBM, kBK,
-                       CU_TENSOR_MAP_SWIZZLE_NONE);
+    ok = tensor_map_2d(&ta.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.M, p.K, p.sak * 4, kBM,
+                       kBK, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (ok) {
     if (NS == 4)  // two TF32 planes: rows of 32 x 4 bytes, 128-byte swizzle
       ok = tensor_map_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes, k_pad,
@@ -904,20 +1058,19 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
                          CU_TENSOR_MAP_SWIZZLE_64B);
   }
   if (!ok) return HML_STATUS_CUDA_ERROR;
-  TcArgs args;
   args.p = p;
   args.split = c.split_k;
   const int kchunks = k_pad / kChunkK;
   args.kc = ((kchunks + c.split_k - 1) / c.split_k) * kChunkK;
   TcPlan plan;
-  if (!tc_plan(BN, NS, c.stages, &plan)) return HML_STATUS_INVALID_VALUE;
+  if (!tc_plan(BN, NS, c.stages, &plan, AM)) return HML_STATUS_INVALID_VALUE;
   args.sa = plan.sa;
   args.so = plan.so;
   args.n_pad = n_pad;
   args.err = err;
   args.bexp = bexp;
-  const size_t smem = tc_plan_bytes(BN, NS, plan);
-  void (*kern)(CUtensorMap, CUtensorMap, TcArgs) = tc_kernel<BN, NS, AK>;
+  const size_t smem = tc_plan_bytes(BN, NS, plan, AM);
+  void (*kern)(AMaps<AM>, CUtensorMap, TcArgs) = tc_kernel<BN, NS, AM>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e == cudaSuccess && c.split_k > 8)
@@ -944,7 +1097,7 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
 // as a second grid with K split across the idle SMs (disjoint rows of C, so
 // the results are those of split_k = 2..8 on those rows).  One CTA per SM:
 // M = 65536, N = 32 is 3 full waves of 148 tiles and 68 more.
-template <int BN, int NS, bool AK>
+template <int BN, int NS, int AM>
 hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
                            const __nv_bfloat16 *planes, int k_pad, int n_pad, int *err,
                            cudaStream_t s) {
@@ -953,10 +1106,10 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
   const int64_t full = (tiles / slots) * slots;
   const int64_t rest = tiles - full;
   if (c.split_k != 1 || n_pad != BN || full == 0 || rest == 0 || 2 * rest > slots)
-    return launch_tc_planes<BN, NS, AK>(p, c, planes, k_pad, n_pad, err, s);
+    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, err, s);
   int split = 1;
   while (split < 8 && 2 * split * rest <= slots && k_pad / (2 * split) >= 4 * kChunkK) split *= 2;
-  if (split == 1) return launch_tc_planes<BN, NS, AK>(p, c, planes, k_pad, n_pad, err, s);
+  if (split == 1) return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, err, s);
   const int64_t m1 = full * kBM;
   GemmProblem head = p, tail = p;
   head.M = static_cast<int>(m1);
@@ -965,9 +1118,9 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
   tail.C = p.C + m1 * p.scm;
   hml_sgemm_config ct = c;
   ct.split_k = split;
-  hml_status st = launch_tc_planes<BN, NS, AK>(head, c, planes, k_pad, n_pad, err, s);
+  hml_status st = launch_tc_planes<BN, NS, AM>(head, c, planes, k_pad, n_pad, err, s);
   if (st != HML_STATUS_SUCCESS) return st;
-  return launch_tc_planes<BN, NS, AK>(tail, ct, planes, k_pad, n_pad, err, s);
+  return launch_tc_planes<BN, NS, AM>(tail, ct, planes, k_pad, n_pad, err, s);
 }
 
 // B -> BF16 planes in `planes` ([NS][n_pad][k_pad]).
@@ -1002,7 +1155,7 @@ hml_status split_b_fh(const GemmProblem &p, void *planes, int *bexp, int k_pad, 
   return HML_STATUS_SUCCESS;
 }
 
-template <int BN, int NS, bool AK>
+template <int BN, int NS, int AM>
 hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s, bool waves) {
   const int k_pad = ((p.K + kChunkK - 1) / kChunkK) * kChunkK;
   const int n_pad = ((p.N + BN - 1) / BN) * BN;
@@ -1019,22 +1172,22 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
     int *bexp = reinterpret_cast<int *>(static_cast<uint8_t *>(ws) + planes_total);
     st = split_b_fh(p, ws, bexp, k_pad, n_pad, s);
     if (st != HML_STATUS_SUCCESS) return st;
-    return launch_tc_planes<BN, NS, AK>(p, c, planes, k_pad, n_pad, device_error_word(), s,
+    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s,
                                         bexp);
   } else {
     st = split_b<NS>(p, planes, k_pad, n_pad, s);
     if (st != HML_STATUS_SUCCESS) return st;
     if (waves)
-      return launch_tc_waves<BN, NS, AK>(p, c, planes, k_pad, n_pad, device_error_word(), s);
-    return launch_tc_planes<BN, NS, AK>(p, c, planes, k_pad, n_pad, device_error_word(), s);
+      return launch_tc_waves<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s);
+    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s);
   }
 }
 
 template <int BN, int NS>
 hml_status run_tc_layout(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s,
                          bool waves) {
-  return p.a_kcontig() ? run_tc<BN, NS, true>(p, c, s, waves)
-                       : run_tc<BN, NS, false>(p, c, s, waves);
+  return p.a_kcontig() ? run_tc<BN, NS, kAK>(p, c, s, waves)
+                       : run_tc<BN, NS, kAM>(p, c, s, waves);
 }
 
 template <int NS>
@@ -1050,6 +1203,11 @@ hml_status run_tc_ns(const GemmProblem &p, const hml_sgemm_config &c, cudaStream
 }
 
 bool aligned16(const void *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
+
+template <int BN>
+hml_status run_tc_unaligned(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s) {
+  return p.a_kcontig() ? run_tc<BN, 3, kAKU>(p, c, s, true) : run_tc<BN, 3, kAMU>(p, c, s, true);
+}
 
 }  // namespace
 
@@ -1080,7 +1238,8 @@ hml_status check_tc(const GemmProblem &p, const hml_sgemm_config &c) {
     return HML_STATUS_INVALID_VALUE;
   if (c.stages < 2 || c.stages > 8) return HML_STATUS_INVALID_VALUE;
   if (!tc_config_fits(c.tile_n, tc_ns(c.algo), c.stages)) return HML_STATUS_INVALID_VALUE;
-  // the A ring is reused for the split-K partial tile
+  // the A ring is reused for the split-K partial tile (an unaligned A's ring
+  // always holds one: launch_tc_unaligned)
   if (c.split_k > 1 &&
       static_cast<size_t>(kBM) * c.tile_n * 4 > static_cast<size_t>(c.stages) * tc_a_bytes())
     return HML_STATUS_INVALID_VALUE;
@@ -1101,6 +1260,32 @@ hml_status launch_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream
     case HML_ALGO_BF16X6: return run_tc_ns<3>(p, c, s, waves);
     case HML_ALGO_FP16X3: return run_tc_ns<5>(p, c, s, waves);
     default: return run_tc_ns<4>(p, c, s, waves);
+  }
+}
+
+// The unaligned form (BF16X6): any 4-byte aligned A with unit stride one way,
+// M and K at least 4, and a stride TMA can encode (4 lines below 2^40 bytes).
+bool tc_unaligned_ok(const GemmProblem &p) {
+  const int64_t ld = p.a_kcontig() ? p.sam : p.sak;
+  return (p.a_kcontig() ? p.sak == 1 : p.sam == 1) && p.M >= 4 && p.K >= 4 && p.N >= 1 &&
+         (reinterpret_cast<uintptr_t>(p.A) & 3u) == 0 && ld >= 1 && ld * 16 < (int64_t(1) << 40);
+}
+
+hml_status launch_tc_unaligned(const GemmProblem &p, const hml_sgemm_config &cfg,
+                               cudaStream_t s) {
+  if (!tc_unaligned_ok(p) || cfg.algo != HML_ALGO_BF16X6) return HML_STATUS_NOT_SUPPORTED;
+  hml_sgemm_config c = cfg;
+  TcPlan pl;
+  // the ring of the aligned form, at least the 64 KB of the widest tile, less
+  // what its wider slots leave no room for
+  c.stages = std::max(c.stages, 4);
+  while (c.stages > 2 && !tc_plan(c.tile_n, 3, c.stages, &pl, kAKU)) c.stages -= 2;
+  switch (c.tile_n) {
+    case 16: return run_tc_unaligned<16>(p, c, s);
+    case 32: return run_tc_unaligned<32>(p, c, s);
+    case 64: return run_tc_unaligned<64>(p, c, s);
+    case 128: return run_tc_unaligned<128>(p, c, s);
+    default: return HML_STATUS_INVALID_VALUE;
   }
 }
 
@@ -1903,7 +2088,7 @@ size_t noalloc_bytes_needed(const GemmProblem &p, const hml_sgemm_config &c) {
 
 // The launch of run_tc with the B planes in the static array and the static
 // error word.
-template <int BN, int NS, bool AK>
+template <int BN, int NS, int AM>
 hml_status run_tc_static(const GemmProblem &p, const hml_sgemm_config &c, const NoAllocAddrs &a,
                          cudaStream_t s) {
   const int k_pad = ((p.K + kChunkK - 1) / kChunkK) * kChunkK;
@@ -1911,7 +2096,7 @@ hml_status run_tc_static(const GemmProblem &p, const hml_sgemm_config &c, const 
   auto *planes = static_cast<__nv_bfloat16 *>(a.scratch);
   hml_status st = split_b<NS>(p, planes, k_pad, n_pad, s);
   if (st != HML_STATUS_SUCCESS) return st;
-  return launch_tc_planes<BN, NS, AK>(p, c, planes, k_pad, n_pad, a.err, s);
+  return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, a.err, s);
 }
 
 template <int NS>
@@ -1919,14 +2104,14 @@ hml_status run_tc_static_ns(const GemmProblem &p, const hml_sgemm_config &c,
                             const NoAllocAddrs &a, cudaStream_t s) {
   const bool ak = p.a_kcontig();
   switch (c.tile_n) {
-    case 16: return ak ? run_tc_static<16, NS, true>(p, c, a, s)
-                       : run_tc_static<16, NS, false>(p, c, a, s);
-    case 32: return ak ? run_tc_static<32, NS, true>(p, c, a, s)
-                       : run_tc_static<32, NS, false>(p, c, a, s);
-    case 64: return ak ? run_tc_static<64, NS, true>(p, c, a, s)
-                       : run_tc_static<64, NS, false>(p, c, a, s);
-    case 128: return ak ? run_tc_static<128, NS, true>(p, c, a, s)
-                        : run_tc_static<128, NS, false>(p, c, a, s);
+    case 16: return ak ? run_tc_static<16, NS, kAK>(p, c, a, s)
+                       : run_tc_static<16, NS, kAM>(p, c, a, s);
+    case 32: return ak ? run_tc_static<32, NS, kAK>(p, c, a, s)
+                       : run_tc_static<32, NS, kAM>(p, c, a, s);
+    case 64: return ak ? run_tc_static<64, NS, kAK>(p, c, a, s)
+                       : run_tc_static<64, NS, kAM>(p, c, a, s);
+    case 128: return ak ? run_tc_static<128, NS, kAK>(p, c, a, s)
+                        : run_tc_static<128, NS, kAM>(p, c, a, s);
     default: return HML_STATUS_INVALID_VALUE;
   }
 }

@@ -109,7 +109,12 @@ const char *hml_version(void);
  * the SMs idle, the rows of that last wave run as a second grid with K split
  * across the idle SMs (those rows then carry split-K rounding, within the
  * same error bounds; hml_sgemm_ex_config runs a configuration exactly as
- * given).  Replaces the launch half of
+ * given).  A problem whose A (the operand of the longer dimension) TMA cannot
+ * address as it stands -- a base or leading dimension that is not a multiple
+ * of 16 bytes -- runs as BF16X6 through four strided views of A where that is
+ * faster than the SIMT tiles; hml_sgemm_ex_config, which runs configurations
+ * as given, refuses the tensor-core ones for such an A, and
+ * hml_sgemm_select reports a configuration that it takes.  Replaces the launch half of
  * hmlSgemm (src/hml_sgemm.cu:120-211 in the reference), generalised to
  * both storage orders, transposes and leading dimensions. */
 hml_status hml_sgemm_ex(hml_order order, hml_op transA, hml_op transB, int M,
