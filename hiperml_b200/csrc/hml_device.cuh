@@ -88,6 +88,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Whether the phase with the given parity has completed (does not suspend).
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Waits for the phase with the given parity to complete, for at most
 // kWaitLimitNs (plus one suspend slice).  Returns false (and records `code`)
 // when the limit expires.
@@ -101,6 +114,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
       return false;
     }
   }
+}
+
+// Waits for phases of two barriers, their first polls overlapping.
+__device__ __forceinline__ bool mbar_wait2(uint64_t *bar0, uint32_t parity0, uint64_t *bar1,
+                                           uint32_t parity1, int *err, int code) {
+  const bool r0 = mbar_test(bar0, parity0), r1 = mbar_test(bar1, parity1);
+  return (r0 || mbar_wait(bar0, parity0, err, code)) && (r1 || mbar_wait(bar1, parity1, err, code));
 }
 
 // ------------------------------------------------- dependent launches

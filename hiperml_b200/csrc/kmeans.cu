@@ -12,10 +12,10 @@
 // (||c_k||^2 - 2 x . c_k), and the dot products of every point with every
 // centroid are one skinny GEMM S = X C^T (points x clusters), in one of three
 // forms:
-//   * tensor-core (method 3, the default where it applies: dims a multiple of
-//     4 up to 64, at most 256 centroids): TF32X3 products on tcgen05 into
-//     TMEM, the argmin read back from the accumulator by the thread that owns
-//     the point;
+//   * tensor-core (method 3, the default wherever its kernel can run: at most
+//     256 centroids that fit in shared memory as BF16 planes): BF16X3 products
+//     on tcgen05 into TMEM, the argmin read back from the accumulator by the
+//     thread that owns the point;
 //   * tiled (method 1, the default otherwise up to 256 dimensions): a
 //     register-tiled FP32 SIMT GEMM with the argmin in its epilogue;
 //   * SGEMM (method 2, wider points): the library's SGEMM in an FP32-accurate
@@ -24,15 +24,17 @@
 // The products carry rounding errors that the reference's direct sums do
 // not, so the pick is made exact: with g_k = ||c_k||^2 - 2 S_k, every
 // centroid whose g_k lies within a bound of the smallest (16 gamma_{dims+4}
-// (||x||^2 + max_k ||c_k||^2) for the FP32 forms, twice that for TF32X3: more
-// than twice the sum of the worst-case errors of g and of the reference's
-// dist) is a candidate, and the reference's choice is always among them.  A
-// point with more than one candidate (or non-finite values) goes to a
-// close-call list that a settle kernel resolves with the reference's own
+// (||x||^2 + max_k ||c_k||^2) for the FP32 forms, 2^-15 of it more for the
+// BF16X3 products: more than twice the sum of the worst-case errors of g and
+// of the reference's dist) is a candidate, and the reference's choice is
+// always among them.  A point with more than one candidate (or non-finite
+// values) goes to a close-call list that is settled with the reference's own
 // arithmetic over the candidates, the first smallest in increasing k.  So
 // every point gets the reference kernel's index, exact ties included.
+#include <algorithm>
 #include <cfloat>
 #include <cstring>
+#include <type_traits>
 
 #include "hml_device.cuh"
 #include "hml_internal.h"
@@ -50,8 +52,7 @@ constexpr int kNormWarps = 8;
 constexpr int kKmeansTiledMaxDims = 256;
 
 // ||c_k||^2 for every centroid, one warp per centroid (FP32; used only to
-// screen candidates).  It runs first in every form, so it also empties the
-// close-call list of the call.
+// screen candidates).  It also empties the close-call list of the call.
 __global__ void centroid_norms_kernel(const float *cent, int k, int d, float *cnorm,
                                       unsigned *ccount) {
   const int lane = threadIdx.x & 31;
@@ -189,7 +190,6 @@ constexpr int64_t kSettleSmemFloats = 96 * 1024 / 4;
 __global__ void __launch_bounds__(256) kmeans_settle_kernel(
     const float *points, int d, const float *cent, int k, const float *cnorm,
     const unsigned *ccount, const uint2 *citems, uint32_t *out, unsigned *exact, int staged) {
-  wait_prior_grid();  // launched as a programmatic dependent of the screening kernel
   extern __shared__ float s_set[];
   const unsigned n = *ccount;
   if (exact && n && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(exact, n);
@@ -623,301 +623,478 @@ __global__ void __launch_bounds__(kTThreads, 2) kmeans_resident_kernel(
 }
 
 // ------------------------------------------------ the tensor-core form
-// (method 3)  The dot products of a 128-point tile with all (up to 256)
-// centroids as TF32X3 products on the tensor cores: x = xh + xl and
-// c = ch + cl with xh = tf32(x), xl = tf32(x - xh) (22 significant bits
-// together), and x.c ~ xh.ch + xh.cl + xl.ch accumulated in FP32 in TMEM.
-// One CTA per SM walks the tiles of a persistent grid:
-//   * warp 0, one lane: TMA of the centroids' TF32 planes (split once by
-//     kmeans_tf32_planes_kernel, K-contiguous), resident in shared memory
-//     in the UMMA K-major layout (128-byte swizzle), then of each point tile
-//     (128 rows x 32 dimensions a box, 128-byte swizzle) into a ring;
-//   * W warpgroups take the CTA's tiles round-robin.  Thread m of a group
-//     owns point m of the tile, which is TMEM lane m: it reads the point's
-//     row, forms ||x||^2 (for the bound) and the TF32 planes, writes them
-//     into the group's TMEM A region with tcgen05.st; one elected thread
-//     then issues the group's tcgen05.mma chain (A in TMEM, B from shared
-//     memory, N = the padded number of centroids) into the group's TMEM
-//     accumulator and commits it to the group's mbarrier; the group reads
-//     its rows back with tcgen05.ld and takes the argmin of g_k =
-//     ||c_k||^2 - 2 x.c_k in increasing k -- the whole row of a point in
-//     one thread, so no merge.  W groups keep W tiles in flight, W issuing
-//     threads in parallel (one thread issues a tcgen05.mma only every ~130
-//     cycles).
-// Close calls go to the close-call list, the margin being twice the SIMT
-// forms' (32 gamma_{dims+4}), as the
-// products' error is up to about four times a direct FP32 sum's (the split
-// leaves 2^-22 per operand; the tensor core's accumulation truncates).
-constexpr int kTcMaxD = 64;    // dimensions (padded to 32)
-constexpr int kTcMaxK = 256;   // centroids (padded to 32): one MMA's N
-constexpr int kTcBox = kTP * 32 * 4;  // bytes of one 128 x 32 FP32 box
+// (method 3, and the automatic choice wherever the centroids fit in shared
+// memory)  One persistent CTA per SM screens 128-point tiles on tcgen05 and
+// settles its own close calls; nothing runs before or after it.
+//
+// Products.  x = x0 + x1 and -2c = c0 + c1 in BF16 (16 significant bits each)
+// and -2 x.c ~ x0.c0 + x0.c1 + x1.c0 accumulated in FP32 in TMEM.  This only
+// screens: the split leaves out at most 3.02 2^-18 |x_j c_j| of a product (so
+// 3.02 2^-18 (||x||^2 + ||c||^2) of a g_k), and a point is settled from the
+// screen only when its second smallest g lies further from the smallest than
+// twice that and the FP32 margin together, 2^-15 + 16 gamma_{dims+4} times
+// ||x||^2 + max ||c||^2 (about the 32 gamma_{dims+4} that TF32X3 products were
+// given before; half their MMAs and half their TMEM).  Every other point gets
+// the reference's own FP32 arithmetic.
+//
+// Roles of a CTA (W = 4 or 2 groups, each with 512 / W TMEM columns: an
+// accumulator of NC columns, then S stages of 32 columns of A):
+//   * controller warp g (one lane): streams group g's tiles, 32 dimensions a
+//     block, into the group's ring of shared-memory slots by TMA (rows that
+//     are not 16-byte aligned through four maps, one per row index modulo 4,
+//     with boxes 4 floats wider, as the SGEMM's unaligned form does), and
+//     issues the group's tcgen05.mma (A in TMEM, the centroid planes resident
+//     in shared memory, N = NC).  A block's slot is refilled when its stage
+//     is written, so the ring needs no barrier of its own for that.
+//   * the 4 warps of group g take the CTA's tiles g, g + W, ...  Thread m owns
+//     point m, which is a TMEM lane: it splits the point's row block by block
+//     into TMEM (tcgen05.st), then -- while the tensor core works on the
+//     tile -- the first blocks of its next tile, then reads the accumulator
+//     row and takes the argmin.
+// With more than 64 centroids (NC columns a pass, P passes) the tile's stages
+// stay in TMEM for all passes.
+//
+// The argmin over a row costs 3 issue slots a centroid (it was 7, and the
+// limit): g in packed FP32x2 adds, the smallest by 3-input minima (half an
+// instruction a value), then the sign bits of g - lim shifted into a mask, in
+// which the first smallest is alone unless the point is a close call.
+// Measured on B200 (whole calls): 1M x 32, k = 64 41 us (65 us with TF32X3
+// products, the per-value argmin and separate prep and settle kernels; 21 us
+// of HBM time), k = 256 109 us (162); 1M x 128, k = 64 90 us (709 us on the
+// tiled form; 84 us of HBM time), 1M x 256, k = 64 171 us (1560; 167); 1M x
+// 11, k = 192 85 us (300).  Wide points are bound by HBM, narrow ones by the
+// groups' own instructions and the latencies between them.
+constexpr int kTcMaxK = 256;                     // centroids (padded to 16)
+constexpr int kTcMaxPlanes = 128 * 1024;         // bytes of the centroids' planes
+constexpr int kTcStageCols = 32;                 // TMEM columns of a 32-dimension block
+__host__ __device__ constexpr int km_slot_bytes(bool au) {
+  return au ? 4 * 36 * 32 * 4 : kTP * 32 * 4;  // 18 KB or 16 KB: a block of a tile
+}
+
+template <bool AU>
+struct KmMaps {
+  CUtensorMap m[AU ? 4 : 1];  // unaligned rows: class r = rows r, r + 4, ...
+};
 
 struct KmTcArgs {
-  int np, d, k, dp, kp, sa;
-  int nc, passes;  // centroids per pass (a multiple of 32) and passes per tile
-  const float *cnorm;
+  const float *points, *cent;
+  int np, d, k;
+  int nb;       // 32-dimension blocks
+  int kp;       // centroids padded to passes x nc
+  int passes, stages, sa;
+  int e[4];     // floats before the data in class r's boxes
   uint32_t *out;
-  unsigned *ccount;
-  uint2 *citems;
+  uint2 *citems;  // [grid][list]: the CTA's close calls
+  int list;       // points a CTA can have
+  unsigned *exact;
   int *err;
 };
 
-// OR of `v` over the 128 threads of a warpgroup (named barrier `id`).
-__device__ __forceinline__ bool group_any(bool v, int id) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred q, %2, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(static_cast<uint32_t>(v)), "r"(id)
-      : "memory");
-  return r != 0;
-}
-
-__device__ __forceinline__ void group_sync(int id) {
-  asm volatile("barrier.cta.sync.aligned %0, 128;" ::"r"(id) : "memory");
-}
-
 __host__ __device__ constexpr int km_tc_threads(int w) { return (4 + 4 * w) * 32; }
 
-template <int W>
+__device__ __forceinline__ uint32_t km_bf16x2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+
+// The values a packed BF16 pair holds.
+__device__ __forceinline__ float2 km_bf16_pair(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// g of 16 consecutive centroids: accumulator columns plus ||c||^2 (at the
+// shared address cn).
+__device__ __forceinline__ void km_g16(const uint32_t (&r)[16], uint32_t cn, float2 *g) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 c = lds128(cn + 16 * i);
+    g[2 * i] = __fadd2_rn(make_float2(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1])),
+                          make_float2(c.x, c.y));
+    g[2 * i + 1] =
+        __fadd2_rn(make_float2(__uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3])),
+                   make_float2(c.z, c.w));
+  }
+}
+
+template <int W, int NC, bool AU>
 __global__ void __launch_bounds__(km_tc_threads(W), 1)
-    kmeans_tc_kernel(const __grid_constant__ CUtensorMap tmX,
-                     const __grid_constant__ CUtensorMap tmB, const __grid_constant__ KmTcArgs a) {
+    kmeans_tc_kernel(const __grid_constant__ KmMaps<AU> tm, const __grid_constant__ KmTcArgs a) {
+  constexpr int SLOT = km_slot_bytes(AU);
+  constexpr int kGroupWarps = 4 * W;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = align_shared(smem_raw, 1024);
-  const int dp = a.dp, kp = a.kp, nkb = dp / 32, SA = a.sa;
-  const int slot = nkb * kTcBox;   // bytes of one point tile
-  const int btile = kp * 128;      // bytes of one (plane, 32-dim block) of the centroids
-  uint8_t *xring = smem;                                  // [SA][nkb][128 x 128 B]
-  uint8_t *bsm = xring + SA * slot;                       // [2][nkb][kp x 128 B]
-  float *cn = reinterpret_cast<float *>(bsm + 2 * nkb * btile);  // [kp]
-  uint64_t *afull = reinterpret_cast<uint64_t *>(cn + kp);
-  uint64_t *aempty = afull + SA;
-  uint64_t *accfull = aempty + SA;  // [W]
-  uint64_t *bfull = accfull + W;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bfull + 1);
-  float *s_cmax = reinterpret_cast<float *>(tmem_slot + 1);
+  const int nb = a.nb, kp = a.kp, SA = a.sa, S = a.stages;
+  const int bblock = kp * 64;  // bytes of one (plane, block) of the centroids
+  uint8_t *xring = smem;                                       // [W][SA][SLOT]
+  uint8_t *bsm = xring + W * SA * SLOT;                        // [2][nb][kp x 64 B]
+  float *cn = reinterpret_cast<float *>(bsm + 2 * nb * bblock);  // [kp]
+  uint64_t *xfull = reinterpret_cast<uint64_t *>(cn + kp);     // [W][SA] block landed
+  uint64_t *sfull = xfull + W * SA;      // [W][S] stage written
+  uint64_t *sempty = sfull + W * S;      // [W][S] the MMAs reading it are done
+  uint64_t *accfull = sempty + W * S;    // [W] a pass's MMAs are done
+  uint64_t *accempty = accfull + W;      // [W] the accumulator is read
+  uint64_t *mmadone = accempty + W;      // every issued MMA has completed
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mmadone + 1);
+  float *s_cmax = reinterpret_cast<float *>(tmem_slot + 1);    // [kGroupWarps]
+  unsigned *s_count = reinterpret_cast<unsigned *>(s_cmax + kGroupWarps);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = (static_cast<int64_t>(a.np) + kTP - 1) / kTP;
   const int my_tiles = static_cast<int>((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  // tiles, and blocks, of group g
+  auto group_tiles = [&](int g) { return my_tiles > g ? (my_tiles - g + W - 1) / W : 0; };
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < SA; ++i) {
-      mbar_init(&afull[i], 1);
-      mbar_init(&aempty[i], 4);  // the 4 warps of the group that read the tile
+    for (int i = 0; i < W * SA; ++i) mbar_init(&xfull[i], 1);
+    for (int i = 0; i < W * S; ++i) {
+      mbar_init(&sfull[i], 4);
+      mbar_init(&sempty[i], 1);
     }
-    for (int g = 0; g < W; ++g) mbar_init(&accfull[g], 1);
-    mbar_init(bfull, 1);
+    for (int g = 0; g < W; ++g) {
+      mbar_init(&accfull[g], 1);
+      mbar_init(&accempty[g], 4);
+    }
+    mbar_init(mmadone, W);
+    *s_count = 0u;
     fence_mbar_init();
-    prefetch_tmap(&tmX);
-    prefetch_tmap(&tmB);
   }
-  // the planes and norms come from the prep kernel launched just before
-  wait_prior_grid();
-  if (warp == 1) {
-    // ||c||^2 (+inf past k: never taken, and never the second smallest) and
-    // its maximum over the centroids
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  __syncthreads();
+
+  // Loads the next block of group g's sequence (its tiles one after another,
+  // round the ring): tile it, block kb, slot `slot`.
+  struct Next {
+    int it = 0, kb = 0, slot = 0, phase = 0;
+  } ld;
+  auto load = [&](int g) {
+    const int64_t t = blockIdx.x + (g + static_cast<int64_t>(ld.it) * W) * gridDim.x;
+    uint64_t *bar = &xfull[g * SA + ld.slot];
+    uint8_t *dst = xring + (g * SA + ld.slot) * SLOT;
+    const int kb = ld.kb;
+    if (++ld.kb == nb) { ld.kb = 0; ++ld.it; }
+    if (++ld.slot == SA) { ld.slot = 0; ld.phase ^= 1; }
+    mbar_arrive_expect_tx(bar, SLOT);
+    if constexpr (AU) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        tma_load_2d(dst + r * (36 * 32 * 4), &tm.m[r], bar, kb * 32,
+                    static_cast<int>(t * (kTP / 4)));
+    } else {
+      tma_load_2d(dst, &tm.m[0], bar, kb * 32, static_cast<int>(t * kTP));
+    }
+  };
+  if (warp < W && lane == 0) {
+    for (const CUtensorMap &m : tm.m) prefetch_tmap(&m);
+    for (int c = 0; c < min(SA, group_tiles(warp) * nb); ++c) load(warp);
+  }
+  if (warp >= 4) {
+    // the centroids' planes (of -2c; K-major, 64-byte swizzle), norms
+    // (+inf past k: never taken) and this warp's largest norm; eight lanes a
+    // centroid, two dimensions each at a time
+    const int sub = lane & 7;
     float cmax = 0.0f;
-    for (int c = lane; c < kp; c += 32) {
-      const float v = c < a.k ? a.cnorm[c] : INFINITY;
-      cn[c] = v;
-      if (c < a.k) cmax = fmaxf(cmax, v);
+    for (int c = 4 * (warp - 4) + (lane >> 3); c < kp; c += 4 * kGroupWarps) {
+      const float *row = a.cent + static_cast<int64_t>(c) * a.d;
+      float sq = 0.0f;
+#pragma unroll 4
+      for (int j = 2 * sub; j < 32 * nb; j += 16) {
+        const float v0 = c < a.k && j < a.d ? row[j] : 0.0f;
+        const float v1 = c < a.k && j + 1 < a.d ? row[j + 1] : 0.0f;
+        sq = fmaf(v0, v0, sq);
+        sq = fmaf(v1, v1, sq);
+        const uint32_t hi = km_bf16x2(-2.0f * v0, -2.0f * v1);
+        const float2 h = km_bf16_pair(hi);
+        const uint32_t lo = km_bf16x2(__fsub_rn(-2.0f * v0, h.x), __fsub_rn(-2.0f * v1, h.y));
+        const int w = (j & 31) >> 1;  // 32-bit word of the 64-byte row
+        const int off = (j >> 5) * bblock + c * 64 + (((w >> 2) ^ ((c >> 1) & 3)) << 4) +
+                        ((w & 3) << 2);
+        *reinterpret_cast<uint32_t *>(bsm + off) = hi;
+        *reinterpret_cast<uint32_t *>(bsm + nb * bblock + off) = lo;
+      }
+      // (kp is a multiple of 16: all lanes of a warp take the same steps)
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (sub == 0) cn[c] = c < a.k ? sq : INFINITY;
+      if (c < a.k) cmax = fmaxf(cmax, sq);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-    if (lane == 0) *s_cmax = cmax;
+    for (int o = 16; o >= 8; o >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+    if (lane == 0) s_cmax[warp - 4] = cmax;
+    fence_proxy_async_smem();  // the MMAs read the planes
   }
-  if (warp == 2) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  const int P = a.passes;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA
+  if (warp < W) {
+    // ---------------------------------------- controller of group `warp`
     if (lane == 0) {
-      mbar_arrive_expect_tx(bfull, 2 * nkb * btile);
-      for (int pl = 0; pl < 2; ++pl)
-        for (int kb = 0; kb < nkb; ++kb)
-          tma_load_2d(bsm + (pl * nkb + kb) * btile, &tmB, bfull, kb * 32, pl * kp);
-      int j = 0;
-      for (; j < my_tiles; ++j) {
-        const int st = j % SA;
-        if (j >= SA && !mbar_wait(&aempty[st], ((j / SA) - 1) & 1, a.err, kDevErrEmptyBarrier))
-          break;
-        const int64_t t = blockIdx.x + static_cast<int64_t>(j) * gridDim.x;
-        mbar_arrive_expect_tx(&afull[st], slot);
-        for (int kb = 0; kb < nkb; ++kb)
-          tma_load_2d(xring + st * slot + kb * kTcBox, &tmX, &afull[st], kb * 32,
-                      static_cast<int>(t * kTP));
+      const int g = warp;
+      const uint32_t tacc = tmem + static_cast<uint32_t>(g * (512 / W));
+      const uint32_t tA = tacc + static_cast<uint32_t>(NC);
+      const uint32_t idesc = idesc_bf16(NC);
+      const int ksteps = (a.d + 15) / 16;
+      const int nt = group_tiles(g);
+      int item = 0;          // passes issued
+      int s = 0, sphase = 0; // the next block's stage
+      // the products of a block against the centroids of pass q
+      auto issue = [&](int stage, int kb, int q, bool fresh) {
+        uint32_t acc = fresh ? 0u : 1u;
+        const uint32_t at = tA + static_cast<uint32_t>(stage * kTcStageCols);
+        const uint64_t b0 = sw64_desc(smem_u32(bsm + kb * bblock + q * NC * 64));
+        const uint64_t b1 = b0 + static_cast<uint64_t>((nb * bblock) >> 4);
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          if (2 * kb + kk >= ksteps) break;  // dimensions past d are zero
+          const uint32_t x0 = at + kk * 8, x1 = x0 + 16;
+          mma_bf16_ts(tacc, x1, b0 + kk * 2, idesc, acc);
+          mma_bf16_ts(tacc, x0, b1 + kk * 2, idesc, 1u);
+          mma_bf16_ts(tacc, x0, b0 + kk * 2, idesc, 1u);
+          acc = 1u;
+        }
+      };
+      bool ok = true;
+      for (int it = 0; it < nt && ok; ++it) {
+        for (int kb = 0; kb < nb && ok; ++kb) {
+          ok = mbar_wait(&sfull[g * S + s], sphase, a.err, kDevErrFullBarrier);
+          if (!ok) break;
+          // the stage is written, so its block's slot has been read
+          if (ld.it < nt) load(g);
+          if (kb == 0 && item > 0)
+            ok = mbar_wait(&accempty[g], (item - 1) & 1, a.err, kDevErrEmptyBarrier);
+          if (!ok) break;
+          tc_fence_after();
+          issue(s, kb, 0, kb == 0);
+          if (P == 1) mma_commit(&sempty[g * S + s]);
+          if (++s == S) { s = 0; sphase ^= 1; }
+        }
+        if (!ok) break;
+        mma_commit(&accfull[g]);
+        ++item;
+        // the other passes, from the same stages (S == nb)
+        for (int q = 1; q < P && ok; ++q, ++item) {
+          ok = mbar_wait(&accempty[g], (item - 1) & 1, a.err, kDevErrEmptyBarrier);
+          if (!ok) break;
+          tc_fence_after();
+          for (int b = 0; b < nb; ++b) issue(b, b, q, b == 0);
+          if (q == P - 1)
+            for (int b = 0; b < nb; ++b) mma_commit(&sempty[g * S + b]);
+          mma_commit(&accfull[g]);
+        }
       }
-      // every load issued has landed before the CTA may exit
-      for (int i = max(0, j - SA); i < j; ++i)
-        mbar_wait(&afull[i % SA], (i / SA) & 1, a.err, kDevErrFullBarrier);
-      mbar_wait(bfull, 0, a.err, kDevErrFullBarrier);
+      mma_commit(mmadone);
+      // every load issued has landed before the ring is reused: the slots
+      // before ld.slot carry this lap's phase, the others the last lap's
+      for (int i = 0; i < SA; ++i)
+        if (i < ld.slot || ld.it * nb + ld.kb >= SA)
+          mbar_wait(&xfull[g * SA + i], i < ld.slot ? ld.phase : ld.phase ^ 1, a.err,
+                    kDevErrFullBarrier);
     }
   } else if (warp >= 4) {
     // ------------------------------------------------- point groups
-    const int g = (warp - 4) >> 2, bar_id = 1 + g;
-    const int m = (warp & 3) * 32 + lane;  // tile row == TMEM lane
-    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const int nc = a.nc, P = a.passes;
-    const uint32_t tacc = tmem + static_cast<uint32_t>(g * (nc + 2 * dp));
-    const uint32_t tA = tacc + static_cast<uint32_t>(nc);  // hi plane dp columns, then lo
-    const bool issuer = warp == 4 + 4 * g && lane == 0;
-    const float cmax = *s_cmax;
+    const int g = (warp - 4) >> 2, w4 = warp & 3;
+    const int m = AU ? 4 * lane + w4 : w4 * 32 + lane;  // the point's row of the tile
+    const uint32_t tacc = tmem + static_cast<uint32_t>(g * (512 / W)) +
+                          (static_cast<uint32_t>(w4 * 32) << 16);  // this warp's lanes
+    const uint32_t tA = tacc + static_cast<uint32_t>(NC);
+    float cmax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kGroupWarps; ++i) cmax = fmaxf(cmax, s_cmax[i]);
     const double nu = (a.d + 4) * 0x1p-24;
-    const float bound = static_cast<float>(32.0 * nu / (1.0 - nu) * 1.001);
-    const uint32_t idesc = idesc_tf32(nc);
-    int it = 0, ph = 0;  // tiles done, phases of accfull[g] done
-    for (int j = g; j < my_tiles; j += W, ++it) {
-      const int st = j % SA;
-      const bool w = mbar_wait(&afull[st], (j / SA) & 1, a.err, kDevErrFullBarrier);
-      if (group_any(!w, bar_id)) break;
-      __syncwarp();  // tcgen05.st is warp-collective
-      // the point's row: ||x||^2 in dimension order, then its TF32 planes
-      const float *xs = reinterpret_cast<const float *>(xring + st * slot);
-      float xn = 0.0f;
-      for (int kb = 0; kb < nkb; ++kb) {
+    const float bound = static_cast<float>((16.0 * nu / (1.0 - nu) + 0x1p-15) * 1.001);
+    [[maybe_unused]] const int e_w = AU ? a.e[w4] : 0;
+
+    // Splits the next block of the group's sequence into its TMEM stage and
+    // adds the block's part of ||x||^2; false when a wait expired.  (The first
+    // lap's wait for a free stage passes: the phase before the first.)
+    int slot = 0, xphase = 0, s = 0, sphase = 0;
+    auto convert = [&](float2 &xn) -> bool {
+      const bool ok = mbar_wait2(&xfull[g * SA + slot], xphase, &sempty[g * S + s], sphase ^ 1,
+                                 a.err, kDevErrFullBarrier);
+      if (!__all_sync(0xffffffffu, ok)) return false;
+      tc_fence_after();
+      const float *xs = reinterpret_cast<const float *>(xring + (g * SA + slot) * SLOT);
+      float2 x[16];
+      if constexpr (AU) {
+        // 36 floats of the lane's row (rows 144 bytes apart), the block's 32
+        // from e_w on
+        const float *row = xs + w4 * (36 * 32) + lane * 36;
+        float y[36];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float x[16];
+        for (int i = 0; i < 9; ++i) {
+          const float4 v = *reinterpret_cast<const float4 *>(row + 4 * i);
+          y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
+        }
+        auto shift = [&](auto e) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float4 v = *reinterpret_cast<const float4 *>(
-                xs + kb * (kTcBox / 4) + m * 32 + (((4 * h + c) ^ (m & 7)) * 4));
-            x[4 * c] = v.x;
-            x[4 * c + 1] = v.y;
-            x[4 * c + 2] = v.z;
-            x[4 * c + 3] = v.w;
-          }
-          uint32_t hi[16], lo[16];
+          for (int i = 0; i < 16; ++i) x[i] = make_float2(y[2 * i + e.value], y[2 * i + 1 + e.value]);
+        };
+        switch (e_w) {  // uniform over the warp
+          case 0: shift(std::integral_constant<int, 0>()); break;
+          case 1: shift(std::integral_constant<int, 1>()); break;
+          case 2: shift(std::integral_constant<int, 2>()); break;
+          default: shift(std::integral_constant<int, 3>()); break;
+        }
+      } else {
+        // row m: 32 floats in 128 bytes, 128-byte swizzle
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            xn = fmaf(x[i], x[i], xn);
-            hi[i] = tf32_rna(x[i]);
-            lo[i] = tf32_rna(__fsub_rn(x[i], __uint_as_float(hi[i])));
-          }
-          const uint32_t col = static_cast<uint32_t>(kb * 32 + h * 16);
-          tmem_st16(tA + lanes + col, hi);
-          tmem_st16(tA + lanes + static_cast<uint32_t>(dp) + col, lo);
+        for (int i = 0; i < 8; ++i) {
+          const float4 v = *reinterpret_cast<const float4 *>(xs + m * 32 + ((i ^ (m & 7)) * 4));
+          x[2 * i] = make_float2(v.x, v.y);
+          x[2 * i + 1] = make_float2(v.z, v.w);
         }
       }
-      // the slot is consumed (every value above was used before this point)
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&aempty[st]);
-      __syncwarp();
+      uint32_t hi[16], lo[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        xn = __ffma2_rn(x[i], x[i], xn);
+        hi[i] = km_bf16x2(x[i].x, x[i].y);
+        const float2 r = __ffma2_rn(km_bf16_pair(hi[i]), make_float2(-1.0f, -1.0f), x[i]);
+        lo[i] = km_bf16x2(r.x, r.y);
+      }
+      const uint32_t dst = tA + static_cast<uint32_t>(s * kTcStageCols);
+      tmem_st16(dst, hi);
+      tmem_st16(dst + 16u, lo);
       tmem_wait_st();
       tc_fence_before();
-      group_sync(bar_id);
-      // the centroids in P passes of nc (the accumulator holds one pass):
-      // argmin of g_k over the point's row, without branches -- g1 the
-      // smallest, k1 the first index reaching it, g2 the second smallest of
-      // the multiset (equal to g1 on a tie; a NaN g makes it g1 too, which
-      // only sends the point to the close-call list)
-      float g1 = INFINITY, g2 = INFINITY;
-      int k1 = 0;
-      bool bad = false;
-      for (int q = 0; q < P; ++q) {
-        if (issuer) {
-          tc_fence_after();
-          bool bok = true;
-          if (it == 0 && q == 0) bok = mbar_wait(bfull, 0, a.err, kDevErrFullBarrier);
-          if (bok) {
-            // products hh, hl, lh of every 8-deep step of every 32-dim block,
-            // against centroids q*nc .. q*nc+nc-1 (rows of the B tiles)
-            for (int kb = 0; kb < nkb; ++kb)
-#pragma unroll
-              for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                for (int pr = 0; pr < 3; ++pr) {
-                  const int ia = pr == 2 ? 1 : 0, jb = pr == 1 ? 1 : 0;
-                  const uint32_t at = tA + static_cast<uint32_t>(ia * dp + kb * 32 + kk * 8);
-                  const uint64_t bd =
-                      sw128_desc(smem_u32(bsm + (jb * nkb + kb) * btile + q * nc * 128)) +
-                      static_cast<uint64_t>((kk * 32) >> 4);
-                  mma_tf32_ts(tacc, at, bd, idesc, (kb | kk | pr) != 0 ? 1u : 0u);
-                }
-          }
-          mma_commit(&accfull[g]);  // arrives once the group's MMAs are done
-        }
-        const bool w2 = mbar_wait(&accfull[g], ph & 1, a.err, kDevErrMmaBarrier);
-        ++ph;
-        if (group_any(!w2, bar_id)) {
-          bad = true;
-          break;
-        }
-        __syncwarp();  // tcgen05.ld is warp-collective
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sfull[g * S + s]);
+      if (++slot == SA) { slot = 0; xphase ^= 1; }
+      if (++s == S) { s = 0; sphase ^= 1; }
+      return true;
+    };
+
+    const int nt = group_tiles(g);
+    // blocks of the next tile split before this tile's argmin: at most what
+    // leaves the stages and the ring a block short of full
+    const int ahead = P > 1 ? 0 : min(nb, min(S - 1, SA));
+    float2 xn = make_float2(0.0f, 0.0f);
+    int done = 0, item = 0;
+    bool ok = true;
+    for (int it = 0; it < nt && ok; ++it) {
+      for (; done < nb && ok; ++done) ok = convert(xn);
+      float2 xnext = make_float2(0.0f, 0.0f);
+      done = 0;
+      if (it + 1 < nt)
+        for (; done < ahead && ok; ++done) ok = convert(xnext);
+      if (!ok) break;
+      const float xsum = xn.x + xn.y + cmax;
+      xn = xnext;
+      // sums near the end of FP32's range: everything is a candidate
+      const float margin = xsum < 1e36f ? bound * xsum + 1e-37f : INFINITY;
+      float g1 = INFINITY;  // the smallest g of the passes so far
+      int k1 = 0;           // its centroid, when the only candidate
+      bool close = true;
+      for (int q = 0; q < P; ++q, ++item) {
+        ok = mbar_wait(&accfull[g], item & 1, a.err, kDevErrMmaBarrier);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         tc_fence_after();
-        for (int c0 = 0; c0 < nc; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld16(tacc + lanes + static_cast<uint32_t>(c0), r);
-          float cv[16];
+        float2 gv[NC / 2];
+        {
+          uint32_t r[NC / 16][16];
 #pragma unroll
-          for (int qq = 0; qq < 4; ++qq) {
-            const float4 v = *reinterpret_cast<const float4 *>(cn + q * nc + c0 + 4 * qq);
-            cv[4 * qq] = v.x;
-            cv[4 * qq + 1] = v.y;
-            cv[4 * qq + 2] = v.z;
-            cv[4 * qq + 3] = v.w;
-          }
+          for (int h = 0; h < NC / 16; ++h) tmem_ld16(tacc + 16 * h, r[h]);
           tmem_wait_ld();
+          const uint32_t cq = smem_u32(cn + q * NC);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float gv = fmaf(-2.0f, __uint_as_float(r[i]), cv[i]);
-            k1 = gv < g1 ? q * nc + c0 + i : k1;
-            g2 = fminf(g2, fmaxf(g1, gv));
-            g1 = fminf(g1, gv);
-          }
+          for (int h = 0; h < NC / 16; ++h) km_g16(r[h], cq + 64 * h, gv + 8 * h);
         }
-        tc_fence_before();  // the reads are done before the next MMAs
-        if (q + 1 < P) group_sync(bar_id);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&accempty[g]);
+        // the pass's smallest (minima skip a NaN g, whose distance the
+        // reference never takes either)
+        float mc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) mc[i] = fminf(gv[i].x, gv[i].y);
+#pragma unroll
+        for (int i = 4; i < NC / 2; ++i) mc[i & 3] = min3(mc[i & 3], gv[i].x, gv[i].y);
+        const float m0 = fminf(min3(mc[0], mc[1], mc[2]), mc[3]);
+        // the candidates, from the signs of g - lim: centroid i of the pass
+        // is bit 31 - i % 32 of word i / 32
+        const float nl = -(m0 + margin);
+        uint32_t half[NC / 16] = {};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int h = 0; h < NC / 16; ++h) {
+            const float2 t = __fadd2_rn(gv[8 * h + i], make_float2(nl, nl));
+            half[h] = __funnelshift_l(__float_as_uint(t.x), half[h], 1);
+            half[h] = __funnelshift_l(__float_as_uint(t.y), half[h], 1);
+          }
+        int cand = 0, kq = 0;
+#pragma unroll
+        for (int h = NC / 16 - 1; h >= 0; --h) {
+          cand += __popc(half[h]);
+          if (half[h]) kq = q * NC + 16 * h + __clz(half[h]) - 16;
+        }
+        // union with the passes before: alone only where the other side's
+        // smallest lies beyond the margin
+        if (m0 + margin < g1) {
+          g1 = m0;
+          k1 = kq;
+          close = cand != 1;
+        } else {
+          close = close || !(g1 + margin < m0);
+          g1 = fminf(g1, m0);
+        }
       }
-      if (bad) break;
-      const int64_t t = blockIdx.x + static_cast<int64_t>(j) * gridDim.x;
-      const int64_t p = t * kTP + m;
+      if (!ok) break;
+      const int64_t p = (blockIdx.x + (g + static_cast<int64_t>(it) * W) * gridDim.x) * kTP + m;
       const bool live = p < a.np;
-      const float lim = g1 + bound * (xn + cmax) + 1e-37f;
-      const bool close = live && !(g2 > lim);
+      const float lim = g1 + margin;
+      close = live && (close || !(lim < INFINITY));
       if (live && !close) a.out[p] = static_cast<uint32_t>(k1);
-      push_close(a.ccount, a.citems, p, lim, close);
+      const unsigned vote = __ballot_sync(0xffffffffu, close);
+      if (vote) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(s_count, static_cast<unsigned>(__popc(vote)));
+        base = __shfl_sync(0xffffffffu, base, 0) + __popc(vote & ((1u << lane) - 1u));
+        if (close)
+          a.citems[static_cast<int64_t>(blockIdx.x) * a.list + base] =
+              make_uint2(static_cast<uint32_t>(p), __float_as_uint(lim));
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
-  // the settle kernel may now be scheduled (it waits for this grid itself);
-  // earlier, its waiting CTAs would sit beside this kernel's on every SM
-  allow_dependent_launch();
-  if (warp == 2) {
+  if (warp == 1) {
+    // the TMEM is freed only once every issued MMA has completed
+    if (lane == 0) mbar_wait(mmadone, 0, a.err, kDevErrMmaBarrier);
+    __syncwarp();
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
-}
-
-// Prep for the tensor-core form: the TF32 planes of the centroids and their
-// norms (one warp per centroid row, the norm summed lane-wise -- it only
-// enters the bound), and an empty close-call list.
-__global__ void kmeans_tc_prep_kernel(const float *cent, int k, int d, int kp, int dp,
-                                      uint32_t *planes, float *cnorm, unsigned *ccount) {
-  allow_dependent_launch();
-  if (blockIdx.x == 0 && threadIdx.x == 0) *ccount = 0u;
-  const int lane = threadIdx.x & 31;
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (c >= kp) return;
-  float sq = 0.0f;
-  for (int j = lane; j < dp; j += 32) {
-    const float v = (c < k && j < d) ? cent[static_cast<int64_t>(c) * d + j] : 0.0f;
-    const uint32_t hi = tf32_rna(v);
-    planes[c * dp + j] = hi;
-    planes[kp * dp + c * dp + j] = tf32_rna(__fsub_rn(v, __uint_as_float(hi)));
-    sq = fmaf(v, v, sq);
+  // ------------------------------------- the CTA's close calls
+  const unsigned n = *s_count;
+  if (n == 0) return;
+  if (a.exact && threadIdx.x == 0) atomicAdd(a.exact, n);
+  // the centroids in FP32 over the ring and the planes, padded rows of d + 1
+  float *cs = reinterpret_cast<float *>(smem);
+  for (int c = warp; c < a.k; c += km_tc_threads(W) / 32)
+    for (int j = lane; j < a.d; j += 32) cs[c * (a.d + 1) + j] = a.cent[static_cast<int64_t>(c) * a.d + j];
+  __syncthreads();
+  if (warp < 4) return;
+  float *xs = cs + a.k * (a.d + 1) + (warp - 4) * a.d;
+  for (unsigned i = warp - 4; i < n; i += kGroupWarps) {
+    const uint2 it = a.citems[static_cast<int64_t>(blockIdx.x) * a.list + i];
+    const float *x = a.points + static_cast<int64_t>(it.x) * a.d;
+    for (int j = lane; j < a.d; j += 32) xs[j] = x[j];
+    __syncwarp();
+    const uint32_t pick = exact_pick_smem(xs, a.d, cs, a.k, cn, __uint_as_float(it.y));
+    if (lane == 0) a.out[it.x] = pick;
+    __syncwarp();  // xs is rewritten for the warp's next entry
   }
-  sq = warp_sum(sq);
-  if (lane == 0 && c < k) cnorm[c] = sq;
 }
 
 // The call's workspace (the stream's second slot): `extra` bytes for the
@@ -945,7 +1122,7 @@ hml_status km_workspace(size_t extra, int np, int k, cudaStream_t s, KmWs *w) {
   return HML_STATUS_SUCCESS;
 }
 
-// ||c||^2 and an empty close-call list; first in every form.
+// ||c||^2 and an empty close-call list; first in the SIMT and SGEMM forms.
 hml_status launch_norms(const float *cent, int k, int d, const KmWs &w, cudaStream_t s) {
   count_launch();
   const int nb = std::min((k + kNormWarps - 1) / kNormWarps, 4 * sm_count());
@@ -956,10 +1133,10 @@ hml_status launch_norms(const float *cent, int k, int d, const KmWs &w, cudaStre
   return cuda_status(e);
 }
 
-// The close calls the screening kernel listed; last in every form
-// (`early`: as a programmatic dependent of a screening kernel that allows it).
+// The close calls the screening kernel listed; last in the SIMT and SGEMM
+// forms.
 hml_status launch_settle(const float *points, int d, const float *cent, int k, const KmWs &w,
-                         uint32_t *out, unsigned *exact, cudaStream_t s, bool early = false) {
+                         uint32_t *out, unsigned *exact, cudaStream_t s) {
   // the centroids, norms and point rows in shared memory when they fit
   const int staged = settle_smem_floats(k, d) <= kSettleSmemFloats ? 1 : 0;
   const size_t smem = staged ? static_cast<size_t>(settle_smem_floats(k, d)) * 4 : 0;
@@ -968,7 +1145,7 @@ hml_status launch_settle(const float *points, int d, const float *cent, int k, c
     e = cudaFuncSetAttribute(kmeans_settle_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(smem));
   if (e == cudaSuccess)
-    e = launch_k_ex(kmeans_settle_kernel, dim3(2 * sm_count()), dim3(256), smem, s, 1, early,
+    e = launch_k_ex(kmeans_settle_kernel, dim3(2 * sm_count()), dim3(256), smem, s, 1, false,
                     points, d, cent, k, static_cast<const float *>(w.cnorm),
                     static_cast<const unsigned *>(w.ccount),
                     static_cast<const uint2 *>(w.citems), out, exact, staged);
@@ -1066,101 +1243,136 @@ hml_status assign_gemm(const float *points, int np, int d, const float *cent, in
   return launch_settle(points, d, cent, k, w, out, exact, s);
 }
 
-// The tensor-core form applies to points with 4 <= dims <= 64 (a multiple of
-// 4, rows 16-byte aligned, for TMA) and at most 256 centroids.
-bool tc_form_applies(const float *points, int d, int k) {
-  return d >= 4 && d % 4 == 0 && (reinterpret_cast<uintptr_t>(points) & 15u) == 0 &&
-         ((d + 31) & ~31) <= kTcMaxD && ((k + 31) & ~31) <= kTcMaxK;
+// Rows that TMA addresses as they stand: whole 16-byte granules.
+bool km_rows_aligned(const float *points, int d) {
+  return d % 4 == 0 && (reinterpret_cast<uintptr_t>(points) & 15u) == 0;
 }
 
-template <int W>
-hml_status launch_km_tc(const CUtensorMap &tx, const CUtensorMap &tb, const KmTcArgs &a,
-                        int grid, size_t smem, cudaStream_t s) {
-  auto kern = kmeans_tc_kernel<W>;
+// What method 3 accepts: points with 4 <= dims <= 64 (a multiple of 4, rows
+// 16-byte aligned) and at most 256 centroids.
+bool tc_form_applies(const float *points, int d, int k) {
+  return d >= 4 && km_rows_aligned(points, d) && d <= 64 && k <= kTcMaxK;
+}
+
+// How the tensor-core kernel runs a shape; false when it cannot.
+struct KmTcPlan {
+  int W, nb, kp, nc, passes, stages, sa;
+  bool au;
+  size_t smem;
+};
+bool km_tc_plan(const float *points, int np, int d, int k, KmTcPlan *out) {
+  KmTcPlan p;
+  p.au = !km_rows_aligned(points, d);
+  // (four row classes; a smaller n leaves a class without a row to address)
+  if (d < 1 || k < 1 || k > kTcMaxK || (p.au && np < 4) ||
+      (reinterpret_cast<uintptr_t>(points) & 3u) != 0)
+    return false;
+  p.nb = (d + 31) / 32;
+  const size_t slot = km_slot_bytes(p.au);
+  const size_t budget = 220 * 1024;
+  auto planes = [&](int kp) { return static_cast<size_t>(4) * kp * 32 * p.nb; };
+  auto width = [](int n) { return n <= 16 ? 16 : n <= 32 ? 32 : n <= 64 ? 64 : 128; };
+  p.passes = 1;
+  // four groups while an accumulator of 64 columns and two stages serve the
+  // shape (more centroids in passes over up to 64 resident dimensions) and
+  // two slots a group fit beside the planes; else two groups, an accumulator
+  // of 128 columns and four stages
+  p.W = 4;
+  p.nc = std::min(64, width(k));
+  p.passes = (k + p.nc - 1) / p.nc;
+  p.kp = p.passes * p.nc;
+  if ((p.passes > 1 && p.nb > 2) || planes(p.kp) + 8 * slot > budget) {
+    p.W = 2;
+    p.nc = std::max(64, width(k));
+    p.passes = (k + p.nc - 1) / p.nc;
+    p.kp = p.passes * p.nc;
+  }
+  p.stages = std::min(4, (512 / p.W - p.nc) / kTcStageCols);
+  if (p.passes > 1) {
+    if (p.nb > p.stages) return false;
+    p.stages = p.nb;
+  }
+  if (planes(p.kp) > kTcMaxPlanes) return false;
+  p.sa = static_cast<int>(std::min<size_t>(4, (budget - planes(p.kp)) / (p.W * slot)));
+  if (p.sa < 2) return false;
+  const int bars = p.W * (p.sa + 2 * p.stages + 2) + 1;
+  p.smem = 1024 + p.W * p.sa * slot + planes(p.kp) + static_cast<size_t>(p.kp) * 4 + bars * 8 +
+           (1 + 4 * p.W + 1) * 4 + 16;
+  // the close calls' centroids and point rows reuse the ring and the planes
+  const size_t settle = (static_cast<size_t>(k) * (d + 1) + 4 * p.W * static_cast<size_t>(d)) * 4;
+  if (settle > p.W * p.sa * slot + planes(p.kp) || p.smem > 227 * 1024) return false;
+  p.smem = std::max<size_t>(p.smem, 120 * 1024);  // one CTA per SM: all 512 TMEM columns
+  *out = p;
+  return true;
+}
+
+template <int W, int NC, bool AU>
+hml_status launch_km_tc(const KmMaps<AU> &tm, const KmTcArgs &a, int grid, size_t smem,
+                        cudaStream_t s) {
+  auto kern = kmeans_tc_kernel<W, NC, AU>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
-  if (e == cudaSuccess)
-    e = launch_k_ex(kern, dim3(grid), dim3(km_tc_threads(W)), smem, s, 1, true, tx, tb, a);
+  if (e == cudaSuccess) e = launch_k(kern, dim3(grid), dim3(km_tc_threads(W)), smem, s, 1, tm, a);
   note_cuda_error(e, "kmeans tensor-core");
   return cuda_status(e);
 }
 
-// The tensor-core form (method 3): centroid planes and norms in one prep
-// kernel, then the persistent screening kernel and the settle kernel, each a
-// programmatic dependent of the kernel before it.
-hml_status assign_tc(const float *points, int np, int d, const float *cent, int k,
-                     uint32_t *out, unsigned *exact, cudaStream_t s) {
-  const int dp = (d + 31) & ~31, kp = (k + 31) & ~31, nkb = dp / 32;
-  // W groups, each with nc + 2 dp TMEM columns (a pass's accumulator, the A
-  // planes): the fewest passes P (nc = kp / P, a multiple of 32) that give
-  // the most groups, up to 4
-  int W = 0, P = 1;
-  for (int p = 1; p <= kp / 32; ++p) {
-    if ((kp / 32) % p) continue;
-    const int per = kp / p + 2 * dp;
-    const int w = per <= 128 ? 4 : per <= 256 ? 2 : per <= 512 ? 1 : 0;
-    if (w > W) {
-      W = w;
-      P = p;
-    }
-    if (W == 4) break;
-  }
-  if (W == 0) return HML_STATUS_NOT_SUPPORTED;
-  const size_t pbytes = static_cast<size_t>(2) * kp * dp * sizeof(uint32_t);
-  KmWs w;
-  hml_status st = km_workspace(pbytes, np, k, s, &w);
+template <bool AU>
+hml_status assign_tc_rows(const KmTcPlan &p, const float *points, int np, int d,
+                          const float *cent, int k, uint32_t *out, unsigned *exact,
+                          cudaStream_t s) {
+  const int64_t tiles = (static_cast<int64_t>(np) + kTP - 1) / kTP;
+  const int grid = static_cast<int>(std::min<int64_t>(tiles, sm_count()));
+  KmTcArgs a = {};
+  a.list = static_cast<int>((tiles + grid - 1) / grid) * kTP;
+  void *ws = nullptr;
+  hml_status st =
+      workspace_slot(1, static_cast<size_t>(grid) * a.list * sizeof(uint2), s, &ws);
   if (st != HML_STATUS_SUCCESS) return st;
-  uint32_t *planes = reinterpret_cast<uint32_t *>(w.extra);
-  count_launch();
-  kmeans_tc_prep_kernel<<<(kp + 7) / 8, 256, 0, s>>>(cent, k, d, kp, dp, planes, w.cnorm,
-                                                     w.ccount);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    note_cuda_error(e, "kmeans prep");
-    return HML_STATUS_CUDA_ERROR;
-  }
-  CUtensorMap tx, tb;
-  memset(&tx, 0, sizeof(tx));
-  memset(&tb, 0, sizeof(tb));
-  if (!tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, points, d, np,
-                     static_cast<uint64_t>(d) * 4, 32, kTP, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !tensor_map_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes, dp, 2 * kp,
-                     static_cast<uint64_t>(dp) * 4, 32, kp, CU_TENSOR_MAP_SWIZZLE_128B))
-    return HML_STATUS_CUDA_ERROR;
-  const size_t slot = static_cast<size_t>(nkb) * kTcBox;
-  const size_t bbytes = static_cast<size_t>(2) * nkb * kp * 128;
-  // a multiple of W (tiles go to group j % W and slot j % sa: each group
-  // then waits for every phase of its slots in order)
-  int sa = static_cast<int>(std::min<size_t>(6, (200 * 1024 - bbytes) / slot));
-  sa -= sa % W;
-  if (sa < 2) return HML_STATUS_NOT_SUPPORTED;
-  size_t smem = 1024 + sa * slot + bbytes + static_cast<size_t>(kp) * 4 +
-                static_cast<size_t>(2 * sa + W + 1) * 8 + 16;
-  // one CTA per SM: each allocates all 512 TMEM columns
-  smem = std::max<size_t>(smem, 120 * 1024);
-  KmTcArgs a;
+  a.points = points;
+  a.cent = cent;
   a.np = np;
   a.d = d;
   a.k = k;
-  a.dp = dp;
-  a.kp = kp;
-  a.sa = sa;
-  a.nc = kp / P;
-  a.passes = P;
-  a.cnorm = w.cnorm;
+  a.nb = p.nb;
+  a.kp = p.kp;
+  a.passes = p.passes;
+  a.stages = p.stages;
+  a.sa = p.sa;
   a.out = out;
-  a.ccount = w.ccount;
-  a.citems = w.citems;
+  a.citems = static_cast<uint2 *>(ws);
+  a.exact = exact;
   a.err = device_error_word();
-  const int64_t tiles = (static_cast<int64_t>(np) + kTP - 1) / kTP;
-  const int grid = static_cast<int>(std::min<int64_t>(tiles, sm_count()));
-  switch (W) {
-    case 4: st = launch_km_tc<4>(tx, tb, a, grid, smem, s); break;
-    case 2: st = launch_km_tc<2>(tx, tb, a, grid, smem, s); break;
-    default: st = launch_km_tc<1>(tx, tb, a, grid, smem, s); break;
+  KmMaps<AU> tm;
+  memset(&tm, 0, sizeof tm);
+  if constexpr (AU) {
+    for (int r = 0; r < 4; ++r) {
+      const float *first = points + static_cast<int64_t>(r) * d;
+      a.e[r] = static_cast<int>((reinterpret_cast<uintptr_t>(first) & 15u) / 4);
+      if (!tensor_map_2d(&tm.m[r], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, first - a.e[r], d + a.e[r],
+                         (np - r + 3) / 4, static_cast<uint64_t>(d) * 16, 36, 32,
+                         CU_TENSOR_MAP_SWIZZLE_NONE))
+        return HML_STATUS_CUDA_ERROR;
+    }
+  } else if (!tensor_map_2d(&tm.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, points, d, np,
+                            static_cast<uint64_t>(d) * 4, 32, kTP, CU_TENSOR_MAP_SWIZZLE_128B)) {
+    return HML_STATUS_CUDA_ERROR;
   }
-  if (st != HML_STATUS_SUCCESS) return st;
-  return launch_settle(points, d, cent, k, w, out, exact, s, true);
+  if (p.W == 2)
+    return p.nc == 64 ? launch_km_tc<2, 64, AU>(tm, a, grid, p.smem, s)
+                      : launch_km_tc<2, 128, AU>(tm, a, grid, p.smem, s);
+  return p.nc == 16   ? launch_km_tc<4, 16, AU>(tm, a, grid, p.smem, s)
+         : p.nc == 32 ? launch_km_tc<4, 32, AU>(tm, a, grid, p.smem, s)
+                      : launch_km_tc<4, 64, AU>(tm, a, grid, p.smem, s);
+}
+
+// The tensor-core form (method 3).
+hml_status assign_tc(const float *points, int np, int d, const float *cent, int k,
+                     uint32_t *out, unsigned *exact, cudaStream_t s) {
+  KmTcPlan p;
+  if (!km_tc_plan(points, np, d, k, &p)) return HML_STATUS_NOT_SUPPORTED;
+  return p.au ? assign_tc_rows<true>(p, points, np, d, cent, k, out, exact, s)
+              : assign_tc_rows<false>(p, points, np, d, cent, k, out, exact, s);
 }
 
 }  // namespace
@@ -1175,7 +1387,9 @@ hml_status kmeans_assign(const float *points, int np, int d, const float *cent, 
     return HML_STATUS_NOT_SUPPORTED;
   if (method == 3 && !tc_form_applies(points, d, k)) return HML_STATUS_NOT_SUPPORTED;
   if (method == 0) {
-    method = tc_form_applies(points, d, k) ? 3 : d <= kKmeansTiledMaxDims ? 1 : 2;
+    // the tensor-core kernel wherever it can run the shape
+    KmTcPlan plan;
+    method = km_tc_plan(points, np, d, k, &plan) ? 3 : d <= kKmeansTiledMaxDims ? 1 : 2;
     if (method == 2 && static_cast<size_t>(k) * sizeof(float) > 200 * 1024) method = 1;
   }
   switch (method) {
