@@ -286,6 +286,24 @@ struct TcArgs {
 };
 
 // ------------------------------------------------------------ B planes
+// How the threads of a splitting kernel walk B's (n, 8-deep k) chunks:
+// consecutive threads along its contiguous dimension, so that whole sectors
+// are read.  (Along k always, an N-contiguous 4096 x 128 B took 5.3 us, 4.1
+// along n; the B of 56 uneven problems 22 us, now 16.)  32-bit indices: 2^32
+// chunks would be planes of 200 GB.
+struct SplitWalk {
+  bool nfast;
+  unsigned inner, chunks;
+  __device__ SplitWalk(int64_t sbk, int64_t sbn, int n_pad, int k_pad)
+      : nfast(sbn == 1 && sbk != 1), inner(nfast ? n_pad : k_pad / 8),
+        chunks(static_cast<unsigned>(n_pad) * (k_pad / 8)) {}
+  __device__ __forceinline__ void at(unsigned c, int *n, int *k0) const {
+    const unsigned o = c / inner, i = c - o * inner;
+    *n = static_cast<int>(nfast ? i : o);
+    *k0 = static_cast<int>(nfast ? o : i) * 8;
+  }
+};
+
 // planes[p][n][k] (k contiguous, zero padded to n_pad x k_pad): NS BF16
 // planes, or for NS = 4 two 32-bit TF32 planes, hi = TF32(x) and
 // lo = TF32(x - hi).
@@ -295,11 +313,11 @@ __global__ void split_b_kernel(const float *B, int64_t sbk, int64_t sbn, int K, 
   // the tensor-core kernel that reads the planes is launched as a
   // programmatic dependent: its set-up and A loads overlap this kernel
   allow_dependent_launch();
-  const int64_t chunks = static_cast<int64_t>(n_pad) * (k_pad / 8);
-  for (int64_t c = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; c < chunks;
-       c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int n = static_cast<int>(c / (k_pad / 8));
-    const int k0 = static_cast<int>(c % (k_pad / 8)) * 8;
+  const SplitWalk walk(sbk, sbn, n_pad, k_pad);
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < walk.chunks;
+       c += gridDim.x * blockDim.x) {
+    int n, k0;
+    walk.at(c, &n, &k0);
     float x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -1317,14 +1335,16 @@ struct TcBatchProblem {
   int64_t scm, scn;
   int M, N;
   float alpha, beta;
-  int akc;    // 1: A is K-contiguous (128 x 32 boxes, 128-byte swizzle)
-  int cpt;    // 64-deep chunks of K (K padded to 64)
   int n_pad;  // rows of one B plane
-  int pad_;
 };
 
 struct TcBatchItem {
-  int prob, tm, tn, pad_;
+  int prob, tm, tn;
+  int cpt_akc;  // 2 * (64-deep chunks of K) + (A is K-contiguous): the
+                // problem's, beside the tile so that a role that takes the
+                // item waits for no further load
+  __host__ __device__ int cpt() const { return cpt_akc >> 1; }
+  __host__ __device__ bool akc() const { return cpt_akc & 1; }
 };
 
 struct TcBatchArgs {
@@ -1344,7 +1364,19 @@ struct TcBatchArgs {
 // sa + so blocks (<= 16) plus NI chunks (<= 4).
 constexpr int kItemRing = 32;
 constexpr int kNoItem = -1;  // the sentinel published once the queue is empty
-constexpr int kQueueAhead = 4;  // queue indices a CTA's producer takes ahead
+// Queue indices a CTA's producer takes before it has loaded the item before
+// them.  After an item of 16 chunks or more none: the round trips of the index
+// and the record (about 1 us each) hide behind the ring the item leaves full.
+// Shorter ones need some ahead, but never more than half a round of the items
+// left, or the CTAs that start first take all of a short queue (four ahead
+// always: 148 tiles of K = 4096 took 262 us, four after one another on 37 SMs;
+// 78 now; 60 uneven problems 862 us, 329 with this order alone).
+constexpr int kQueueAhead = 4;
+__device__ __forceinline__ int queue_ahead(int cpt, unsigned taken, unsigned nitems) {
+  const int want = cpt >= 16 ? 0 : cpt >= 8 ? 2 : kQueueAhead;
+  const unsigned left = taken < nitems ? nitems - taken : 0u;
+  return min(want, static_cast<int>(left / (2 * gridDim.x)));
+}
 
 // A role's walk through the items its CTA takes, in the order taken: item j
 // of the sequence is read from ring slot j % kItemRing once published, and
@@ -1379,7 +1411,7 @@ struct QueueCursor {
   // boundary; false when a wait expired.
   __device__ __forceinline__ bool next(const TcBatchArgs &a, uint64_t *ifull, uint64_t *iempty,
                                        const TcBatchItem *ring, bool warp_role, int lane) {
-    if (++c < pr->cpt) return true;
+    if (++c < it.cpt()) return true;
     ++j;
     return fetch(a, ifull, iempty, ring, warp_role, lane);
   }
@@ -1465,17 +1497,15 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
     // loads its A blocks; a sentinel ends every role's walk
     if (lane == 0) {
       int blk = 0;
-      // the indices of the next kQueueAhead items are taken ahead and the
-      // record of the next one is loaded ahead, so the atomics' and the
-      // load's round trips overlap the current item's loads (a CTA holds at
-      // most kQueueAhead - 1 items it has not started: at the end of the
-      // longest-first queue, short ones)
+      // q[0 .. w-1]: the indices taken ahead, q[0] the next item's
       unsigned q[kQueueAhead];
 #pragma unroll
-      for (int i = 0; i < kQueueAhead; ++i) q[i] = atomicAdd(&args.queue[0], 1u);
+      for (int i = 0; i < kQueueAhead; ++i) q[i] = 0u;
+      q[0] = atomicAdd(&args.queue[0], 1u);
+      int w = 1;
       const unsigned nitems = static_cast<unsigned>(args.nitems);
-      TcBatchItem nxt = {kNoItem, 0, 0, 0};
-      if (q[0] < nitems) nxt = args.items[q[0]];
+      const TcBatchItem none = {kNoItem, 0, 0, 0};
+      TcBatchItem nxt = q[0] < nitems ? args.items[q[0]] : none;
       for (int j = 0;; ++j) {
         const int r = j % kItemRing;
         if (!mbar_wait(&iempty[r], ((j / kItemRing) & 1) ^ 1, args.err, kDevErrEmptyBarrier))
@@ -1484,17 +1514,21 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
         iring[r] = it;
         mbar_arrive(&ifull[r]);  // release: the slot's item is visible to the waiters
         if (it.prob == kNoItem) break;
-        // slide the window: one more index taken, the next record loaded
+        // slide the window and fill it up again (past the end: harmless)
+        const int depth = queue_ahead(it.cpt(), q[0], nitems);
 #pragma unroll
         for (int i = 0; i + 1 < kQueueAhead; ++i) q[i] = q[i + 1];
-        q[kQueueAhead - 1] = atomicAdd(&args.queue[0], 1u);  // past the end: harmless
-        nxt = {kNoItem, 0, 0, 0};
-        if (q[0] < nitems) nxt = args.items[q[0]];
-        const TcBatchProblem &pr = args.probs[it.prob];
+        --w;
+#pragma unroll
+        for (int i = 0; i < kQueueAhead; ++i)
+          if (i >= w && i < depth) q[i] = atomicAdd(&args.queue[0], 1u);
+        w = max(w, depth);
+        const bool known = w > 0;
         const CUtensorMap *tm = args.tmA + it.prob;
         const int m0 = it.tm * kBM;
+        const int blocks = it.cpt() * P;
         bool ok = true;
-        for (int kq = 0; kq < pr.cpt * P && ok; ++kq, ++blk) {
+        for (int kq = 0; kq < blocks && ok; ++kq, ++blk) {
           const int k0 = kq * kBK;
           const int s = blk % SA;
           if (!mbar_wait(&aempty[s], ((blk / SA) & 1) ^ 1, args.err, kDevErrEmptyBarrier)) {
@@ -1503,12 +1537,22 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
           }
           mbar_arrive_expect_tx(&afull[s], A32_BYTES);
           // k beyond K (the last chunk of a problem) reads TMA's zero fill
-          if (pr.akc)
+          if (it.akc())
             tma_load_2d(aring + s * A32_BYTES, tm, &afull[s], k0, m0);
           else
             tma_load_2d(aring + s * A32_BYTES, tm, &afull[s], m0, k0);
+          if (known && kq == 1) {  // (an item has at least two blocks)
+            // the next item's record and map, behind the loads just issued
+            nxt = q[0] < nitems ? args.items[q[0]] : none;
+            if (nxt.prob != kNoItem) prefetch_tmap(args.tmA + nxt.prob);
+          }
         }
         if (!ok) break;
+        if (!known) {
+          q[0] = atomicAdd(&args.queue[0], 1u);
+          w = 1;
+          nxt = q[0] < nitems ? args.items[q[0]] : none;
+        }
       }
       // every atomic taken ahead has returned (its register is read) before
       // this thread's arrival on the finish counter, so the last CTA's reset
@@ -1605,7 +1649,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       if (!__all_sync(0xffffffffu, w)) break;
       const float *a32 = reinterpret_cast<const float *>(aring + s * A32_BYTES);
       float x[32];
-      if (cur.pr->akc) {
+      if (cur.it.akc()) {
         // row m holds 32 floats in 128 bytes, 128-byte swizzle
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -1673,7 +1717,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&accempty[b]);
-      if (cur.c == cur.pr->cpt - 1) {
+      if (cur.c == cur.it.cpt() - 1) {
         // the item's last chunk: C tile (row m, columns d*DC ..) and reset
         const TcBatchProblem &pr = *cur.pr;
         const int64_t gm = static_cast<int64_t>(cur.it.tm) * kBM + m;
@@ -1728,11 +1772,11 @@ template <int NS>
 __global__ void split_b_batch_kernel(const TcSplitDesc *descs) {
   allow_dependent_launch();  // the tensor-core kernels wait for the planes
   const TcSplitDesc d = descs[blockIdx.y];
-  const int64_t chunks = static_cast<int64_t>(d.n_pad) * (d.k_pad / 8);
-  for (int64_t c = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; c < chunks;
-       c += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int n = static_cast<int>(c / (d.k_pad / 8));
-    const int k0 = static_cast<int>(c % (d.k_pad / 8)) * 8;
+  const SplitWalk walk(d.sbk, d.sbn, d.n_pad, d.k_pad);
+  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < walk.chunks;
+       c += gridDim.x * blockDim.x) {
+    int n, k0;
+    walk.at(c, &n, &k0);
     float x[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -1840,8 +1884,9 @@ hml_status tc_batch_create(const GemmProblem *probs, int count, cudaStream_t str
     if (tm > 0x7fffffff) return HML_STATUS_NOT_SUPPORTED;
     for (int64_t x = 0; x < tm; ++x)
       for (int64_t y = 0; y < tn; ++y)
-        items[cls[i]].push_back({k_pad[i] / kChunkK, TcBatchItem{i, static_cast<int>(x),
-                                                                 static_cast<int>(y), 0}});
+        items[cls[i]].push_back({k_pad[i] / kChunkK,
+                                 TcBatchItem{i, static_cast<int>(x), static_cast<int>(y),
+                                             k_pad[i] / kChunkK * 2 + (p.a_kcontig() ? 1 : 0)}});
   }
   // per class: the items longest first, the order the queue hands them out
   // (each CTA takes the next when it can: longest-processing-time first)
@@ -1914,8 +1959,6 @@ hml_status tc_batch_create(const GemmProblem *probs, int count, cudaStream_t str
     q.N = p.N;
     q.alpha = p.alpha;
     q.beta = p.beta;
-    q.akc = p.a_kcontig() ? 1 : 0;
-    q.cpt = k_pad[i] / kChunkK;
     q.n_pad = n_pad[i];
     hs[i] = TcSplitDesc{p.B, p.sbk, p.sbn, p.K, p.N, k_pad[i], n_pad[i], planes};
   }
@@ -1977,7 +2020,8 @@ hml_status tc_batch_launch(const TcBatch *b, cudaStream_t s) {
   // each tile kernel is a programmatic dependent of the kernel before it:
   // its CTAs start on the SMs that kernel has finished with, and only its B
   // loader waits for that kernel to complete
-  for (int c = 0; c < 3 && e == cudaSuccess; ++c) {
+  // (the widest class, whose tiles take longest, first)
+  for (int c = 2; c >= 0 && e == cudaSuccess; --c) {
     const TcBatch::Class &k = b->cls[c];
     if (k.grid == 0) continue;
     if (c == 0)
