@@ -738,19 +738,13 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
 #pragma unroll
         for (int k = 0; k < 32; ++k) x[k] = a32[k * kBM + m];
       }
-      // consume the values (the first plane's split reads every one) before
-      // the warp releases the slot: one lane arrives for the warp, and
-      // __syncwarp alone does not wait for the other lanes' shared-memory
-      // loads to return
       uint32_t wv[16];
       [[maybe_unused]] uint32_t wl[16];
       [[maybe_unused]] int sexp_m = 0;
       if constexpr (TF) {
-        // hi of the first 16 values; the other 16 only need to have arrived
+        // hi of the first 16 values
 #pragma unroll
         for (int k = 0; k < 16; ++k) wv[k] = tf32_rna(x[k]);
-#pragma unroll
-        for (int k = 16; k < 32; ++k) asm volatile("" ::"f"(x[k]));
       } else if constexpr (FH) {
         // the row's scale for this block from its largest magnitude, then
         // both planes
@@ -760,8 +754,6 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
       } else {
         split_plane32<NS == 1>(x, wv);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&aempty[s]);
       // the A stage: wait until the MMAs that read it are done
       w = mbar_wait(&opempty[o], ((kb / SO) & 1) ^ 1, args.err, kDevErrEmptyBarrier);
       if (!__all_sync(0xffffffffu, w)) {
@@ -778,6 +770,15 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         if (lane == 0) mbar_arrive(&sfull[kb % R]);
       }
       const uint32_t dst = tA + lanes + static_cast<uint32_t>(o * SC);
+      // The slot is released after the first TMEM store, which takes (every
+      // lane's) words of values read from all of it: a __syncwarp before the
+      // arrival neither waits for the other lanes' loads to return nor keeps
+      // their use from being scheduled behind it, and TMA refills the slot at
+      // once (a build with registers to spare did so, and lost rows).
+      auto release = [&]() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&aempty[s]);
+      };
       if constexpr (TF) {
         // one TF32 per column: plane hi in columns 0..31 (k), lo in 32..63;
         // lo = TF32(x - hi), the residual being exact in FP32
@@ -787,6 +788,7 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
 #pragma unroll
         for (int k = 0; k < 16; ++k) wv[k] = tf32_rna(x[16 + k]);
         tmem_st16(dst + 16u, wv);
+        release();
 #pragma unroll
         for (int k = 0; k < 16; ++k) x[16 + k] -= __uint_as_float(wv[k]);
 #pragma unroll
@@ -797,9 +799,11 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         tmem_st16(dst + 48u, wv);
       } else if constexpr (FH) {
         tmem_st16(dst, wv);
+        release();
         tmem_st16(dst + 16u, wl);
       } else {
         tmem_st16(dst, wv);
+        release();
         split_plane32<NS == 2>(x, wv);
         tmem_st16(dst + 16u, wv);
         if constexpr (NS == 3) {
@@ -1662,13 +1666,13 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       }
       uint32_t wv[16];
       split_plane32<NS == 1>(x, wv);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&aempty[s]);
       w = mbar_wait(&opempty[o], ((blk / SO) & 1) ^ 1, args.err, kDevErrEmptyBarrier);
       if (!__all_sync(0xffffffffu, w)) break;
       tc_fence_after();
       const uint32_t dst = tA + lanes + static_cast<uint32_t>(o * SC);
       tmem_st16(dst, wv);
+      __syncwarp();  // every lane's values are in: see the single-problem kernel
+      if (lane == 0) mbar_arrive(&aempty[s]);
       split_plane32<NS == 2>(x, wv);
       tmem_st16(dst + 16u, wv);
       if constexpr (NS == 3) {
