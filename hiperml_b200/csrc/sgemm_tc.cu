@@ -160,6 +160,24 @@ __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
   return r;
 }
 
+// Releasing a shared-memory slot for the warp takes every lane's values to be
+// in: a __syncwarp before one lane's arrival neither waits for the other
+// lanes' loads to return nor keeps their use from being scheduled behind it,
+// and TMA refills the slot at once (a build with registers to spare did so,
+// and lost rows).  A slot is released after the block's first TMEM store,
+// which takes words of values from all of the row -- except in a ring of 2
+// slots (EARLY), which cannot wait for the operand stage that store needs
+// (8192^3 5.95 ms, 6.58 with the later release): there the arriving lane
+// comes from a vote on words w computed from every value.
+template <int N>
+__device__ __forceinline__ void release_early(uint64_t *bar, const uint32_t (&w)[N], int lane) {
+  uint32_t all = w[0];
+#pragma unroll
+  for (int i = 1; i < N; ++i) all |= w[i];
+  const uint32_t vote = __ballot_sync(0xffffffffu, all != 0x5bd1e995u);
+  if (lane == (vote ? __ffs(vote) - 1 : 0)) mbar_arrive(bar);
+}
+
 template <int NS>
 __device__ __forceinline__ void pack8(const float (&x)[8], uint4 (&out)[NS]) {
   uint32_t w[NS][4];
@@ -281,6 +299,12 @@ struct TcArgs {
   int sa, so;      // A ring and operand-stage depths
   int n_pad;       // rows of one B plane in the workspace
   int e[4];        // unaligned A: floats before the data in class r's boxes
+  // persistent form: `whole` tiles run whole, tile t by CTA t % gridDim.x, then
+  // `tail` tiles split in K over `tsplit` CTAs each (K ranges of tkc)
+  int64_t whole;
+  int tail, tsplit, tkc;
+  float *partial;      // [tail * tsplit][BN][kBM], a CTA's K range of its tail tile
+  unsigned *arrivals;  // [tail], zero between launches
   int *err;
   const int *bexp;  // FP16X3: per column of B, the scale exponent S_n of its planes
 };
@@ -426,10 +450,13 @@ __host__ __device__ constexpr size_t tc_b_bytes(int bn, int ns) {
 // FP16X3: the ring of per-row scale exponents the converters hand to the
 // drain warps, one entry per K block in flight (2 x the operand stages).
 __host__ __device__ constexpr int tc_fh_ring(int so) { return 2 * so; }
+// Scratch of the persistent form's drain warps (a row each of plain sums).
+constexpr size_t kPersistScratch = 8 * 64 * 4 + 16;
 size_t tc_plan_bytes(int bn, int ns, const TcPlan &pl, int am = kAM) {
   const size_t ring = ns == 5 ? static_cast<size_t>(tc_fh_ring(pl.so)) * (8 + kBM * 4) : 0;
   return 1024 + pl.sa * tc_a_bytes(am) + pl.so * tc_b_bytes(bn, ns) +
-         8 * (2 * pl.sa + 2 * pl.so + 2 * 4 + 1) + 16 + ring + 16;
+         8 * (2 * pl.sa + 2 * pl.so + 2 * 4 + 1) + 16 + ring + 16 +
+         (am_unaligned(am) ? kPersistScratch : 0);
 }
 
 // The deepest operand-stage ring that fits TMEM and shared memory next to
@@ -455,7 +482,13 @@ __host__ __device__ constexpr uint32_t tc_tmem_alloc_cols(int bn, int ns, int so
   return tc_pow2_cols(tc_issuers(bn, ns) * bn + so * tc_stage_cols(ns));
 }
 
-template <int BN, int NS, int AM>
+// PERSIST: one CTA per SM walks several tiles ("segments" of its work), the
+// loads, conversions and MMAs of the next running on while the drain warps
+// finish a tile, so a tile's set-up, first loads and drain (9 to 12 us a tile
+// otherwise, of about 60 at K = 4096) are paid once.  Consecutive CTAs take
+// consecutive tiles, all at about the same K, so they share operands in L2.
+// Which problems run so, and what it measured: tc_walk.
+template <int BN, int NS, int AM, bool PERSIST, bool EARLY>
 __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
     tc_kernel(const __grid_constant__ AMaps<AM> tmA, const __grid_constant__ CUtensorMap tmB,
               TcArgs args) {
@@ -508,6 +541,9 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
   int *bad_flag = reinterpret_cast<int *>(tmem_slot + 1);
   int *tmax_sh = bad_flag + 1;        // FP16X3: the largest column scale exponent of the tile
   int *sexp = align_shared(tmax_sh + 1, 16);  // [R][kBM]
+  // PERSIST: whether the CTA arrived last at a tail tile; the drain warps' rows
+  [[maybe_unused]] int *last_flag = tmax_sh;
+  [[maybe_unused]] float *scratch = reinterpret_cast<float *>(sexp);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = args.split;
@@ -517,8 +553,41 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
   const int kbeg = rank * args.kc;
   const int kend = min(p.K, kbeg + args.kc);
   const int nkb = kend > kbeg ? (kend - kbeg + kBK - 1) / kBK : 0;
-  const int nchunks = (nkb + P - 1) / P;
   const uint32_t tmem_cols = tc_tmem_alloc_cols(BN, NS, SO);
+
+  // The CTA's segments: a tile (first row and column) and a K range in nkb
+  // blocks.  Roles count blocks across segments: with PERSIST a segment has
+  // whole chunks (the last may hold a block of zeros).
+  struct Segment {
+    int64_t m0;
+    int n0, kbeg, kend, nkb;
+    int tile, rank;  // the tail: the tile's index in it (else -1), the K range's
+  };
+  const bool has_tail =
+      PERSIST && static_cast<int64_t>(blockIdx.x) < static_cast<int64_t>(args.tail) * args.tsplit;
+  auto segment = [&](int i, Segment *sg) -> bool {
+    if constexpr (!PERSIST) {
+      *sg = {m0, n0, kbeg, kend, nkb, -1, 0};
+      return i == 0;
+    } else {
+      int64_t t = blockIdx.x + static_cast<int64_t>(i) * gridDim.x;
+      *sg = {0, 0, 0, p.K, 0, -1, 0};
+      if (t >= args.whole) {
+        if (!has_tail || t - blockIdx.x != args.whole) return false;  // (whole waves before it)
+        sg->tile = static_cast<int>(blockIdx.x) / args.tsplit;
+        sg->rank = static_cast<int>(blockIdx.x) % args.tsplit;
+        t = args.whole + sg->tile;
+        sg->kbeg = sg->rank * args.tkc;
+        sg->kend = min(p.K, sg->kbeg + args.tkc);
+      }
+      const int64_t tiles_m = (static_cast<int64_t>(p.M) + kBM - 1) / kBM;
+      sg->m0 = t % tiles_m * kBM;
+      sg->n0 = static_cast<int>(t / tiles_m) * BN;
+      sg->nkb = sg->kend > sg->kbeg ? (sg->kend - sg->kbeg + P * kBK - 1) / (P * kBK) * P : 0;
+      return true;
+    }
+  };
+  Segment sg;
 
   if (tid == 0) {
     for (int s = 0; s < SA; ++s) {
@@ -550,30 +619,34 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
     // -------------------------------------------------------- TMA, A
     if (lane == 0) {
       for (const CUtensorMap &t : tmA.m) prefetch_tmap(&t);
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % SA;
-        if (!mbar_wait(&aempty[s], ((kb / SA) & 1) ^ 1, args.err, kDevErrEmptyBarrier)) {
-          *bad_flag = 1;
-          break;
-        }
-        uint8_t *dst = aring + s * A32_BYTES;
-        const int k0 = kbeg + kb * kBK;
-        mbar_arrive_expect_tx(&afull[s], tc_a_tx(AM));
-        if constexpr (AU) {
-          // class r: rows (columns) r, r + 4, ... of the block, from a
-          // 16-byte boundary; k0 and m0 are multiples of 32
+      bool ok = true;
+      for (int i = 0, base = 0; ok && segment(i, &sg); ++i, base += sg.nkb) {
+        for (int kb = 0; kb < sg.nkb; ++kb) {
+          const int s = (base + kb) % SA;
+          ok = mbar_wait(&aempty[s], (((base + kb) / SA) & 1) ^ 1, args.err, kDevErrEmptyBarrier);
+          if (!ok) {
+            *bad_flag = 1;
+            break;
+          }
+          uint8_t *dst = aring + s * A32_BYTES;
+          const int k0 = sg.kbeg + kb * kBK;
+          mbar_arrive_expect_tx(&afull[s], tc_a_tx(AM));
+          if constexpr (AU) {
+            // class r: rows (columns) r, r + 4, ... of the block, from a
+            // 16-byte boundary; k0 and m0 are multiples of 32
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
-            if (AK)
-              tma_load_2d(dst + r * (36 * 32 * 4), &tmA.m[r], &afull[s], k0,
-                          static_cast<int>(m0 / 4));
-            else
-              tma_load_2d(dst + r * (132 * 8 * 4), &tmA.m[r], &afull[s], static_cast<int>(m0),
-                          k0 / 4);
-        } else if (AK) {  // 128 rows of 32 floats (128-byte swizzle)
-          tma_load_2d(dst, &tmA.m[0], &afull[s], k0, static_cast<int>(m0));
-        } else {  // 32 rows (k) of 128 floats (m)
-          tma_load_2d(dst, &tmA.m[0], &afull[s], static_cast<int>(m0), k0);
+            for (int r = 0; r < 4; ++r)
+              if (AK)
+                tma_load_2d(dst + r * (36 * 32 * 4), &tmA.m[r], &afull[s], k0,
+                            static_cast<int>(sg.m0 / 4));
+              else
+                tma_load_2d(dst + r * (132 * 8 * 4), &tmA.m[r], &afull[s], static_cast<int>(sg.m0),
+                            k0 / 4);
+          } else if (AK) {  // 128 rows of 32 floats (128-byte swizzle)
+            tma_load_2d(dst, &tmA.m[0], &afull[s], k0, static_cast<int>(sg.m0));
+          } else {  // 32 rows (k) of 128 floats (m)
+            tma_load_2d(dst, &tmA.m[0], &afull[s], static_cast<int>(sg.m0), k0);
+          }
         }
       }
     }
@@ -585,18 +658,22 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
       // which may still be running (programmatic dependent launch); nothing
       // else this kernel reads depends on it
       wait_prior_grid();
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int o = kb % SO;
-        if (!mbar_wait(&opempty[o], ((kb / SO) & 1) ^ 1, args.err, kDevErrEmptyBarrier)) {
-          *bad_flag = 1;
-          break;
-        }
-        uint8_t *dst = bring + o * BSLOT;
-        const int k0 = kbeg + kb * kBK;
-        mbar_arrive_expect_tx(&opfull[o], BSLOT);
+      bool ok = true;
+      for (int i = 0, base = 0; ok && segment(i, &sg); ++i, base += sg.nkb) {
+        for (int kb = 0; kb < sg.nkb; ++kb) {
+          const int o = (base + kb) % SO;
+          ok = mbar_wait(&opempty[o], (((base + kb) / SO) & 1) ^ 1, args.err, kDevErrEmptyBarrier);
+          if (!ok) {
+            *bad_flag = 1;
+            break;
+          }
+          uint8_t *dst = bring + o * BSLOT;
+          const int k0 = sg.kbeg + kb * kBK;
+          mbar_arrive_expect_tx(&opfull[o], BSLOT);
 #pragma unroll
-        for (int i = 0; i < PL; ++i)
-          tma_load_2d(dst + i * BPL_BYTES, &tmB, &opfull[o], k0, i * args.n_pad + n0);
+          for (int pl = 0; pl < PL; ++pl)
+            tma_load_2d(dst + pl * BPL_BYTES, &tmB, &opfull[o], k0, pl * args.n_pad + sg.n0);
+        }
       }
     }
   } else if (warp >= 2 && warp < 2 + NI) {
@@ -608,84 +685,88 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
       const int b = warp - 2;
       const uint32_t dacc = tacc + static_cast<uint32_t>(b * BN);
       bool ok = true;
-      for (int q = b; q < nchunks && ok; q += NI) {
-        const bool w =
-            mbar_wait(&accempty[b], ((q / NI) & 1) ^ 1, args.err, kDevErrEmptyBarrier);
-        if (!w) {
-          ok = false;
-          break;
-        }
-        const int kb1 = min(nkb, (q + 1) * P);
-        // the products of block kb whose plane indices sum to t0 .. t1, the
-        // smallest (largest sum) first; `fresh` zeroes the accumulator
-        auto issue = [&](int kb, int t0, int t1, bool fresh) {
-          const int o = kb % SO;
-          const uint32_t astage = tA + static_cast<uint32_t>(o * SC);
-          const uint64_t b_desc = sw64_desc(smem_u32(bring + o * BSLOT));
-          uint32_t acc = fresh ? 0u : 1u;
-#pragma unroll
-          for (int t = PL - 1; t >= 0; --t) {
-            if (t < t0 || t > t1) continue;
-#pragma unroll
-            for (int kk = 0; kk < kBK / KMMA; ++kk)
-#pragma unroll
-              for (int i = 0; i <= t; ++i) {
-                mma_bf16_ts(dacc, astage + static_cast<uint32_t>(i * PLC + kk * 8),
-                            b_desc + static_cast<uint64_t>(((t - i) * BPL_BYTES + kk * 32) >> 4),
-                            IDESC, acc);
-                acc = 1u;
-              }
-          }
-        };
-        for (int kb = q * P; kb < kb1; ++kb) {
-          const int o = kb % SO;
-          const bool first = kb == q * P;
-          const bool w = mbar_wait(&opfull[o], (kb / SO) & 1, args.err, kDevErrFullBarrier);
+      // chunk q of a segment is chunk base / P + q of the CTA
+      for (int i = 0, base = 0; ok && segment(i, &sg); ++i, base += sg.nkb) {
+        for (int q = (b + NI - base / P % NI) % NI; q * P < sg.nkb && ok; q += NI) {
+          const bool w = mbar_wait(&accempty[b], (((base / P + q) / NI) & 1) ^ 1, args.err,
+                                   kDevErrEmptyBarrier);
           if (!w) {
             ok = false;
             break;
           }
-          tc_fence_after();
+          const int kb1 = min(sg.nkb, (q + 1) * P);
+          // the products of block kb whose plane indices sum to t0 .. t1, the
+          // smallest (largest sum) first; `fresh` zeroes the accumulator
+          auto issue = [&](int kb, int t0, int t1, bool fresh) {
+            const int o = (base + kb) % SO;
+            const uint32_t astage = tA + static_cast<uint32_t>(o * SC);
+            const uint64_t b_desc = sw64_desc(smem_u32(bring + o * BSLOT));
+            uint32_t acc = fresh ? 0u : 1u;
+#pragma unroll
+            for (int t = PL - 1; t >= 0; --t) {
+              if (t < t0 || t > t1) continue;
+#pragma unroll
+              for (int kk = 0; kk < kBK / KMMA; ++kk)
+#pragma unroll
+                for (int i = 0; i <= t; ++i) {
+                  mma_bf16_ts(dacc, astage + static_cast<uint32_t>(i * PLC + kk * 8),
+                              b_desc + static_cast<uint64_t>(((t - i) * BPL_BYTES + kk * 32) >> 4),
+                              IDESC, acc);
+                  acc = 1u;
+                }
+            }
+          };
+          for (int kb = q * P; kb < kb1; ++kb) {
+            const int o = (base + kb) % SO;
+            const bool first = kb == q * P;
+            const bool w =
+                mbar_wait(&opfull[o], ((base + kb) / SO) & 1, args.err, kDevErrFullBarrier);
+            if (!w) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            if constexpr (AU) {
+              issue(kb, 1, PL - 1, first);
+              continue;
+            }
+            const uint32_t astage = tA + static_cast<uint32_t>(o * SC);
+            const uint64_t b_desc = TF ? sw128_desc(smem_u32(bring + o * BSLOT))
+                                       : sw64_desc(smem_u32(bring + o * BSLOT));
+#pragma unroll
+            for (int kk = 0; kk < kBK / KMMA; ++kk) {
+#pragma unroll
+              for (int i = 0; i < PL; ++i)
+#pragma unroll
+                for (int j = 0; j < PL - i; ++j) {
+                  // A plane i: PLC columns per plane, 8 per MMA step (16 BF16
+                  // or 8 TF32 deep); B: 32 bytes per step; descriptor start
+                  // addresses count 16-byte units
+                  const uint32_t at = astage + static_cast<uint32_t>(i * PLC + kk * 8);
+                  const uint64_t bd =
+                      b_desc + static_cast<uint64_t>((j * BPL_BYTES + kk * 32) >> 4);
+                  const uint32_t acc = (!first || kk > 0 || i > 0 || j > 0) ? 1u : 0u;
+                  if constexpr (TF)
+                    mma_tf32_ts(dacc, at, bd, IDESC, acc);
+                  else
+                    mma_bf16_ts(dacc, at, bd, IDESC, acc);
+                }
+            }
+            mma_commit(&opempty[o]);
+          }
           if constexpr (AU) {
-            issue(kb, 1, PL - 1, first);
-            continue;
+            // the leading products of the whole chunk last: the tensor core
+            // truncates on every accumulation, so only these 4 of a chunk's 24
+            // lose bits of the full sum (error against FP64 at K = 1501:
+            // 1.2e-7, 5.3e-7 in the order above, 1.8e-7 for the SIMT tiles;
+            // the order above releases a stage earlier, 2 % at N = 128)
+            for (int kb = q * P; ok && kb < kb1; ++kb) {
+              issue(kb, 0, 0, false);
+              mma_commit(&opempty[(base + kb) % SO]);
+            }
           }
-          const uint32_t astage = tA + static_cast<uint32_t>(o * SC);
-          const uint64_t b_desc = TF ? sw128_desc(smem_u32(bring + o * BSLOT))
-                                     : sw64_desc(smem_u32(bring + o * BSLOT));
-#pragma unroll
-          for (int kk = 0; kk < kBK / KMMA; ++kk) {
-#pragma unroll
-            for (int i = 0; i < PL; ++i)
-#pragma unroll
-              for (int j = 0; j < PL - i; ++j) {
-                // A plane i: PLC columns per plane, 8 per MMA step (16 BF16
-                // or 8 TF32 deep); B: 32 bytes per step; descriptor start
-                // addresses count 16-byte units
-                const uint32_t at = astage + static_cast<uint32_t>(i * PLC + kk * 8);
-                const uint64_t bd =
-                    b_desc + static_cast<uint64_t>((j * BPL_BYTES + kk * 32) >> 4);
-                const uint32_t acc = (!first || kk > 0 || i > 0 || j > 0) ? 1u : 0u;
-                if constexpr (TF)
-                  mma_tf32_ts(dacc, at, bd, IDESC, acc);
-                else
-                  mma_bf16_ts(dacc, at, bd, IDESC, acc);
-              }
-          }
-          mma_commit(&opempty[o]);
+          if (ok) mma_commit(&accfull[b]);
         }
-        if constexpr (AU) {
-          // the leading products of the whole chunk last: the tensor core
-          // truncates on every accumulation, so only these 4 of a chunk's 24
-          // lose bits of the full sum (error against FP64 at K = 1501:
-          // 1.2e-7, 5.3e-7 in the order above, 1.8e-7 for the SIMT tiles;
-          // the order above releases a stage earlier, 2 % at N = 128)
-          for (int kb = q * P; ok && kb < kb1; ++kb) {
-            issue(kb, 0, 0, false);
-            mma_commit(&opempty[kb % SO]);
-          }
-        }
-        if (ok) mma_commit(&accfull[b]);
       }
       if (!ok) *bad_flag = 1;
       // tracks every MMA this thread issued
@@ -698,7 +779,9 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
     const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
     // kAKU: TMEM lane 32 w + l holds row 4 l + w (class w) of the tile
     [[maybe_unused]] const int e_w = AM == kAKU ? args.e[warp & 3] : 0;
-    for (int kb = g; kb < nkb; kb += G) {
+    int blocks = 0;  // of all segments
+    for (int i = 0; segment(i, &sg); ++i) blocks += sg.nkb;
+    for (int kb = g; kb < blocks; kb += G) {
       const int s = kb % SA, o = kb % SO;
       bool w = mbar_wait(&afull[s], (kb / SA) & 1, args.err, kDevErrFullBarrier);
       if (!__all_sync(0xffffffffu, w)) {
@@ -754,6 +837,16 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
       } else {
         split_plane32<NS == 1>(x, wv);
       }
+      if constexpr (EARLY) {
+        if constexpr (TF) {
+          uint32_t all[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) all[k] = wv[k] | __float_as_uint(x[16 + k]);
+          release_early(&aempty[s], all, lane);
+        } else {
+          release_early(&aempty[s], wv, lane);
+        }
+      }
       // the A stage: wait until the MMAs that read it are done
       w = mbar_wait(&opempty[o], ((kb / SO) & 1) ^ 1, args.err, kDevErrEmptyBarrier);
       if (!__all_sync(0xffffffffu, w)) {
@@ -770,12 +863,8 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         if (lane == 0) mbar_arrive(&sfull[kb % R]);
       }
       const uint32_t dst = tA + lanes + static_cast<uint32_t>(o * SC);
-      // The slot is released after the first TMEM store, which takes (every
-      // lane's) words of values read from all of it: a __syncwarp before the
-      // arrival neither waits for the other lanes' loads to return nor keeps
-      // their use from being scheduled behind it, and TMA refills the slot at
-      // once (a build with registers to spare did so, and lost rows).
       auto release = [&]() {
+        if (EARLY) return;
         __syncwarp();
         if (lane == 0) mbar_arrive(&aempty[s]);
       };
@@ -836,148 +925,249 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
       for (int o = 16; o > 0; o >>= 1) tmax = max(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
       if (tid == kDrainWarp0 * 32) *tmax_sh = tmax;
     }
-    for (int q = 0; q < nchunks; ++q) {
-      const int b = q % NI;
-      bool w = mbar_wait(&accfull[b], (q / NI) & 1, args.err, kDevErrMmaBarrier);
-      [[maybe_unused]] float mult = 1.0f, mult2 = 1.0f;
-      [[maybe_unused]] bool twostep = false;
-      if constexpr (FH) {
-        // block q's partial of row m is scaled by 2^(S_m,q + S_n): undo the
-        // row's scale and the tile's largest column scale, 2^e.  Outside
-        // the normal range the factor is applied in two exact steps
-        // (2^(e -+ 126), then 2^(+-126)), so no contribution is lost or
-        // clamped that FP32 itself would represent.
-        if (w) w = mbar_wait(&sfull[q % R], (q / R) & 1, args.err, kDevErrFullBarrier);
-        if (w) {
-          const int e = -sexp[(q % R) * kBM + mrow] - tmax;
-          twostep = e < -126 || e > 127;
-          mult = exp2_int(e < -126 ? e + 126 : e > 127 ? e - 126 : e);
-          mult2 = e < -126 ? 0x1p-126f : 0x1p126f;
-        }
-      }
-      if (!__all_sync(0xffffffffu, w)) {  // tcgen05.ld is warp-collective
-        *bad_flag = 1;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t src = tacc + lanes + static_cast<uint32_t>(b * BN + d * DC);
-      if constexpr (FH && DC >= 16) {
-        // up to 32 columns loaded before one wait (16 when the running sums
-        // take 64 registers); packed FP32x2 FMAs
-        constexpr int W = DC >= 64 ? 16 : DC >= 32 ? 32 : DC;
-        const float2 m2 = make_float2(mult, mult), m22 = make_float2(mult2, mult2);
-#pragma unroll
-        for (int c = 0; c < DC; c += W) {
-          uint32_t r0[W];
-#pragma unroll
-          for (int h = 0; h < W; h += 16)
-            tmem_ld16(src + c + h, *reinterpret_cast<uint32_t(*)[16]>(r0 + h));
-          tmem_wait_ld();
-          if (!twostep) {
-#pragma unroll
-            for (int i = 0; i < W; i += 2) {
-              const float2 r = make_float2(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]));
-              const float2 t = __ffma2_rn(r, m2, make_float2(sums[c + i], sums[c + i + 1]));
-              sums[c + i] = t.x;
-              sums[c + i + 1] = t.y;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < W; i += 2) {
-              const float2 r = make_float2(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]));
-              const float2 t = __ffma2_rn(__fmul2_rn(r, m2), m22,
-                                          make_float2(sums[c + i], sums[c + i + 1]));
-              sums[c + i] = t.x;
-              sums[c + i + 1] = t.y;
-            }
+    bool ok = true;
+    for (int i = 0, base = 0; segment(i, &sg); ++i, base += sg.nkb) {
+      for (int q = 0; ok && q * P < sg.nkb; ++q) {
+        const int qc = base / P + q, b = qc % NI;  // chunk of the CTA, its accumulator
+        bool w = mbar_wait(&accfull[b], (qc / NI) & 1, args.err, kDevErrMmaBarrier);
+        [[maybe_unused]] float mult = 1.0f, mult2 = 1.0f;
+        [[maybe_unused]] bool twostep = false;
+        if constexpr (FH) {
+          // block q's partial of row m is scaled by 2^(S_m,q + S_n): undo the
+          // row's scale and the tile's largest column scale, 2^e.  Outside
+          // the normal range the factor is applied in two exact steps
+          // (2^(e -+ 126), then 2^(+-126)), so no contribution is lost or
+          // clamped that FP32 itself would represent.
+          if (w) w = mbar_wait(&sfull[q % R], (q / R) & 1, args.err, kDevErrFullBarrier);
+          if (w) {
+            const int e = -sexp[(q % R) * kBM + mrow] - tmax;
+            twostep = e < -126 || e > 127;
+            mult = exp2_int(e < -126 ? e + 126 : e > 127 ? e - 126 : e);
+            mult2 = e < -126 ? 0x1p-126f : 0x1p126f;
           }
         }
-      } else if constexpr (DC >= 16) {
-#pragma unroll
-        for (int c = 0; c < DC; c += 16) {
-          uint32_t r0[16];
-          tmem_ld16(src + c, r0);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) sums[c + i] += __uint_as_float(r0[i]);
+        ok = __all_sync(0xffffffffu, w);  // tcgen05.ld is warp-collective
+        if (!ok) {
+          *bad_flag = 1;
+          break;
         }
-      } else {
-        static_assert(DC % 8 == 0, "drain width");
-        uint32_t r0[8];
-        tmem_ld8(src, r0);
-        tmem_wait_ld();
-        if constexpr (FH) {
-          if (!twostep) {
+        tc_fence_after();
+        const uint32_t src = tacc + lanes + static_cast<uint32_t>(b * BN + d * DC);
+        if constexpr (FH && DC >= 16) {
+          // up to 32 columns loaded before one wait (16 when the running sums
+          // take 64 registers); packed FP32x2 FMAs
+          constexpr int W = DC >= 64 ? 16 : DC >= 32 ? 32 : DC;
+          const float2 m2 = make_float2(mult, mult), m22 = make_float2(mult2, mult2);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) sums[i] = __fmaf_rn(__uint_as_float(r0[i]), mult, sums[i]);
-          } else {
+          for (int c = 0; c < DC; c += W) {
+            uint32_t r0[W];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-              sums[i] = __fmaf_rn(__fmul_rn(__uint_as_float(r0[i]), mult), mult2, sums[i]);
+            for (int h = 0; h < W; h += 16)
+              tmem_ld16(src + c + h, *reinterpret_cast<uint32_t(*)[16]>(r0 + h));
+            tmem_wait_ld();
+            if (!twostep) {
+#pragma unroll
+              for (int i = 0; i < W; i += 2) {
+                const float2 r = make_float2(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]));
+                const float2 t = __ffma2_rn(r, m2, make_float2(sums[c + i], sums[c + i + 1]));
+                sums[c + i] = t.x;
+                sums[c + i + 1] = t.y;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < W; i += 2) {
+                const float2 r = make_float2(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]));
+                const float2 t = __ffma2_rn(__fmul2_rn(r, m2), m22,
+                                            make_float2(sums[c + i], sums[c + i + 1]));
+                sums[c + i] = t.x;
+                sums[c + i + 1] = t.y;
+              }
+            }
+          }
+        } else if constexpr (DC >= 16) {
+#pragma unroll
+          for (int c = 0; c < DC; c += 16) {
+            uint32_t r0[16];
+            tmem_ld16(src + c, r0);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sums[c + i] += __uint_as_float(r0[i]);
           }
         } else {
+          static_assert(DC % 8 == 0, "drain width");
+          uint32_t r0[8];
+          tmem_ld8(src, r0);
+          tmem_wait_ld();
+          if constexpr (FH) {
+            if (!twostep) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sums[i] += __uint_as_float(r0[i]);
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&accempty[b]);
-    }
-    // ---------------------------------------------------- epilogue
-    // (the running sums stay in this branch's registers; the barrier is the
-    // one every other thread reaches below)
-    __syncthreads();
-    const bool failed = *bad_flag != 0;
-    float *red = reinterpret_cast<float *>(smem);  // [BN][kBM], reuses the A ring
-    const int m = AM == kAKU ? 4 * lane + (warp & 3) : tid & (kBM - 1);  // row of the tile
-    const int64_t gm = m0 + m;
-    if (failed) {
+              for (int i = 0; i < 8; ++i)
+                sums[i] = __fmaf_rn(__uint_as_float(r0[i]), mult, sums[i]);
+            } else {
 #pragma unroll
-      for (int i = 0; i < DC; ++i) sums[i] = 0.0f;
-    }
-    if (split > 1 || AU) {
+              for (int i = 0; i < 8; ++i)
+                sums[i] = __fmaf_rn(__fmul_rn(__uint_as_float(r0[i]), mult), mult2, sums[i]);
+            }
+          } else {
 #pragma unroll
-      for (int i = 0; i < DC; ++i) red[(d * DC + i) * kBM + m] = sums[i];
-      if constexpr (AU) {
-        // an infinite operand (or one that rounds to BF16's infinity) has
-        // NaN in its residual planes: non-finite sums are formed again in
-        // plain FP32, as the SIMT kernels form them, the lanes of the warp
-        // over k
-        bool odd = false;
-#pragma unroll
-        for (int i = 0; i < DC; ++i) odd |= !(fabsf(sums[i]) <= FLT_MAX);
-        __syncwarp();
-        for (unsigned todo = __ballot_sync(0xffffffffu, odd && gm < p.M); todo;
-             todo &= todo - 1) {
-          const int mr = __shfl_sync(0xffffffffu, m, __ffs(todo) - 1);
-          const float *arow = p.A + (m0 + mr) * p.sam;
-          for (int n = n0 + d * DC; n < min(p.N, n0 + (d + 1) * DC); ++n) {
-            if (fabsf(red[(n - n0) * kBM + mr]) <= FLT_MAX) continue;
-            float v = 0.0f;
-            for (int64_t k = kbeg + lane; k < kend; k += 32)
-              v = fmaf(arow[k * p.sak], p.B[k * p.sbk + n * p.sbn], v);
-            v = warp_sum(v);
-            __syncwarp();
-            if (lane == 0) red[(n - n0) * kBM + mr] = v;
+            for (int i = 0; i < 8; ++i) sums[i] += __uint_as_float(r0[i]);
           }
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&accempty[b]);
       }
-    } else if (gm < p.M) {
+      if constexpr (PERSIST) {
+        // ------------------------------------------------ end of a segment
+        // (after a wait that expired no tile is stored)
+        const int m = AM == kAKU ? 4 * lane + (warp & 3) : mrow;  // row of the tile
+        const int64_t gm = sg.m0 + m;
+        const int nb = sg.n0 + d * DC;
+        if constexpr (AU) {
+          // rows with a non-finite sum again in plain FP32 (see below), through
+          // the warp's scratch row
+          bool odd = false;
 #pragma unroll
-      for (int i = 0; i < DC; ++i) {
-        const int gn = n0 + d * DC + i;
-        if (gn < p.N) {
-          float *cp = p.C + gm * p.scm + static_cast<int64_t>(gn) * p.scn;
-          float v = sums[i];
-          if constexpr (FH) v = scale_pow2(v, tmax - args.bexp[gn]);
-          *cp = axpby(p.alpha, v, p.beta, cp);
+          for (int c = 0; c < DC; ++c) odd |= !(fabsf(sums[c]) <= FLT_MAX);
+          float *row = scratch + (warp - kDrainWarp0) * DC;
+          for (unsigned todo = __ballot_sync(0xffffffffu, ok && odd && gm < p.M); todo;
+               todo &= todo - 1) {
+            const int l = __ffs(todo) - 1;
+            const float *arow = p.A + __shfl_sync(0xffffffffu, gm, l) * p.sam;
+            for (int n = nb; n < min(p.N, nb + DC); ++n) {
+              float v = 0.0f;
+              for (int64_t kk = sg.kbeg + lane; kk < sg.kend; kk += 32)
+                v = fmaf(arow[kk * p.sak], p.B[kk * p.sbk + n * p.sbn], v);
+              v = warp_sum(v);
+              if (lane == 0) row[n - nb] = v;
+            }
+            __syncwarp();
+            if (lane == l) {
+#pragma unroll
+              for (int c = 0; c < DC; ++c)
+                if (!(fabsf(sums[c]) <= FLT_MAX) && nb + c < p.N) sums[c] = row[c];
+            }
+            __syncwarp();
+          }
+        }
+        if (sg.tile >= 0) {
+          // a K range of a tail tile, the CTA's last segment: published, and
+          // summed at the end
+          float *part = args.partial + mrow + (static_cast<int64_t>(blockIdx.x) * BN + d * DC) * kBM;
+#pragma unroll
+          for (int c = 0; c < DC; ++c) __stcg(part + c * kBM, sums[c]);
+          __threadfence();
+        } else if (ok && gm < p.M) {
+#pragma unroll
+          for (int c = 0; c < DC; ++c) {
+            if (nb + c < p.N) {
+              float *cp = p.C + gm * p.scm + static_cast<int64_t>(nb + c) * p.scn;
+              *cp = axpby(p.alpha, sums[c], p.beta, cp);
+            }
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < DC; ++c) sums[c] = 0.0f;
+      }
+    }
+    if constexpr (!PERSIST) {
+      // ---------------------------------------------------- epilogue
+      // (the running sums stay in this branch's registers; the barrier is the
+      // one every other thread reaches below)
+      __syncthreads();
+      const bool failed = *bad_flag != 0;
+      float *red = reinterpret_cast<float *>(smem);  // [BN][kBM], reuses the A ring
+      const int m = AM == kAKU ? 4 * lane + (warp & 3) : tid & (kBM - 1);  // row of the tile
+      const int64_t gm = m0 + m;
+      if (failed) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) sums[i] = 0.0f;
+      }
+      if (split > 1 || AU) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) red[(d * DC + i) * kBM + m] = sums[i];
+        if constexpr (AU) {
+          // an infinite operand (or one that rounds to BF16's infinity) has
+          // NaN in its residual planes: non-finite sums are formed again in
+          // plain FP32, as the SIMT kernels form them, the lanes of the warp
+          // over k
+          bool odd = false;
+#pragma unroll
+          for (int i = 0; i < DC; ++i) odd |= !(fabsf(sums[i]) <= FLT_MAX);
+          __syncwarp();
+          for (unsigned todo = __ballot_sync(0xffffffffu, odd && gm < p.M); todo;
+               todo &= todo - 1) {
+            const int mr = __shfl_sync(0xffffffffu, m, __ffs(todo) - 1);
+            const float *arow = p.A + (m0 + mr) * p.sam;
+            for (int n = n0 + d * DC; n < min(p.N, n0 + (d + 1) * DC); ++n) {
+              if (fabsf(red[(n - n0) * kBM + mr]) <= FLT_MAX) continue;
+              float v = 0.0f;
+              for (int64_t k = kbeg + lane; k < kend; k += 32)
+                v = fmaf(arow[k * p.sak], p.B[k * p.sbk + n * p.sbn], v);
+              v = warp_sum(v);
+              __syncwarp();
+              if (lane == 0) red[(n - n0) * kBM + mr] = v;
+            }
+          }
+        }
+      } else if (gm < p.M) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) {
+          const int gn = n0 + d * DC + i;
+          if (gn < p.N) {
+            float *cp = p.C + gm * p.scm + static_cast<int64_t>(gn) * p.scn;
+            float v = sums[i];
+            if constexpr (FH) v = scale_pow2(v, tmax - args.bexp[gn]);
+            *cp = axpby(p.alpha, v, p.beta, cp);
+          }
         }
       }
     }
   }
-  if (warp < kDrainWarp0) __syncthreads();
-  if (split > 1 || AU) {  // an unaligned A's tile always goes through shared memory
+  if constexpr (PERSIST) {
+    if (has_tail) {  // (uniform over the CTA)
+      // The tail tile: the CTA that arrives last sums its K ranges in rank
+      // order, as the cluster does in the other form (no CTA waits for
+      // another); all threads, their roles done, 4 rows each.
+      const int tile = static_cast<int>(blockIdx.x) / args.tsplit;
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        const bool last =
+            atomicAdd(&args.arrivals[tile], 1u) == static_cast<unsigned>(args.tsplit - 1);
+        if (last) args.arrivals[tile] = 0u;  // ready for the next call
+        *last_flag = last && *bad_flag == 0;
+      }
+      __syncthreads();
+      if (*last_flag) {
+        __threadfence();
+        const int64_t t = args.whole + tile;  // n_pad == BN: the tile is its row tile
+        const float4 *part = reinterpret_cast<const float4 *>(
+            args.partial + static_cast<int64_t>(tile) * args.tsplit * BN * kBM);
+        for (int e = tid; e < BN * kBM / 4; e += kThreads) {
+          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+          for (int r = 0; r < args.tsplit; ++r) {
+            const float4 v = __ldcg(part + static_cast<int64_t>(r) * (BN * kBM / 4) + e);
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+          }
+          const float sv[4] = {sum.x, sum.y, sum.z, sum.w};
+          const int n = e * 4 / kBM;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int pos = e * 4 % kBM + j;  // TMEM lane
+            const int64_t gm = t * kBM + (AM == kAKU ? 4 * (pos & 31) + (pos >> 5) : pos);
+            if (gm < p.M && n < p.N) {
+              float *cp = p.C + gm * p.scm + static_cast<int64_t>(n) * p.scn;
+              *cp = axpby(p.alpha, sv[j], p.beta, cp);
+            }
+          }
+        }
+      }
+    }
+  }
+  if (!PERSIST && warp < kDrainWarp0) __syncthreads();
+  if (!PERSIST && (split > 1 || AU)) {  // an unaligned A's tile always goes through shared memory
     [[maybe_unused]] int tmax_all = 0;
     if constexpr (FH) {
       wait_prior_grid();  // the column scale exponents below
@@ -1037,10 +1227,19 @@ bool tc_config_fits(int bn, int ns, int stages) {
 namespace {
 
 // Launch of the kernel with the B planes already split into `planes`.
-template <int BN, int NS, int AM>
+// The persistent form's work: see TcArgs.
+struct TcWalk {
+  int64_t whole = 0;
+  int tail = 0, tsplit = 1;
+  float *partial = nullptr;
+  unsigned *arrivals = nullptr;
+};
+
+template <int BN, int NS, int AM, bool PERSIST = false>
 hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
                             const __nv_bfloat16 *planes, int k_pad, int n_pad, int *err,
-                            cudaStream_t s, const int *bexp = nullptr) {
+                            cudaStream_t s, const int *bexp = nullptr,
+                            const TcWalk *walk = nullptr) {
   if (NS == 5 && !bexp) return HML_STATUS_INVALID_VALUE;
   AMaps<AM> ta;
   CUtensorMap tb;
@@ -1063,8 +1262,8 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
                          ak ? 32 : 8, CU_TENSOR_MAP_SWIZZLE_NONE);
     }
   } else if (AM == kAK)
-    ok = tensor_map_2d(&ta.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.K, p.M, p.sam * 4, kBK, kBM,
-                       CU_TENSOR_MAP_SWIZZLE_128B);
+    ok = tensor_map_2d(&ta.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.K, p.M, p.sam * 4, kBK,
+                       kBM, CU_TENSOR_MAP_SWIZZLE_128B);
   else
     ok = tensor_map_2d(&ta.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.M, p.K, p.sak * 4, kBM,
                        kBK, CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -1085,14 +1284,26 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   const int kchunks = k_pad / kChunkK;
   args.kc = ((kchunks + c.split_k - 1) / c.split_k) * kChunkK;
   TcPlan plan;
-  if (!tc_plan(BN, NS, c.stages, &plan, AM)) return HML_STATUS_INVALID_VALUE;
+  // slots are held until the operand stage is free (release_early): rings of 4
+  // get 6 where that fits (18944 x 64 x 4096, 4 slots: 74.8 us when released
+  // earlier, 77.0, 74.3 with 6), and the persistent form, which only the
+  // automatic choice reaches, has no use for one of 2
+  int sa = c.stages;
+  if (sa == 4 || (PERSIST && sa == 2)) {
+    const int given = sa;
+    for (sa = 6; sa > given && !tc_plan(BN, NS, sa, &plan, AM); sa -= 2) {
+    }
+  }
+  if (!tc_plan(BN, NS, sa, &plan, AM)) return HML_STATUS_INVALID_VALUE;
   args.sa = plan.sa;
   args.so = plan.so;
   args.n_pad = n_pad;
   args.err = err;
   args.bexp = bexp;
   const size_t smem = tc_plan_bytes(BN, NS, plan, AM);
-  void (*kern)(AMaps<AM>, CUtensorMap, TcArgs) = tc_kernel<BN, NS, AM>;
+  void (*kern)(AMaps<AM>, CUtensorMap, TcArgs) =
+      plan.sa == 2 ? tc_kernel<BN, NS, AM, PERSIST, !PERSIST && !am_unaligned(AM)>
+                   : tc_kernel<BN, NS, AM, PERSIST, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e == cudaSuccess && c.split_k > 8)
@@ -1105,6 +1316,15 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   const int64_t tiles_n = n_pad / BN;
   if (tiles_m * c.split_k > 0x7fffffff || tiles_n > 65535) return HML_STATUS_NOT_SUPPORTED;
   dim3 grid(static_cast<unsigned>(tiles_m * c.split_k), static_cast<unsigned>(tiles_n));
+  if constexpr (PERSIST) {
+    args.whole = walk->whole;
+    args.tail = walk->tail;
+    args.tsplit = walk->tsplit;
+    args.tkc = ((kchunks + walk->tsplit - 1) / walk->tsplit) * kChunkK;
+    args.partial = walk->partial;
+    args.arrivals = walk->arrivals;
+    grid = dim3(static_cast<unsigned>(sm_count()));
+  }
   // launched right after split_b_kernel wrote the planes: a programmatic
   // dependent whose B loader waits for it (wait_prior_grid)
   e = launch_k_ex(kern, grid, dim3(tc_warps(BN, NS) * 32), smem, s, c.split_k, true,
@@ -1113,12 +1333,22 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   return cuda_status(e);
 }
 
+// How the last, partial wave of `tiles` row tiles on `slots` SMs is run on the
+// automatic path: split in K so that its tiles take the idle SMs too, when it
+// would leave at least half of them idle (1: as the others).  One CTA per SM:
+// M = 65536, N = 32 is 3 full waves of 148 tiles and 68 more.
+int tail_split(int64_t tiles, int64_t slots, int k_pad) {
+  const int64_t rest = tiles % slots;
+  if (tiles < slots || rest == 0 || 2 * rest > slots) return 1;
+  int split = 1;
+  while (split < 8 && 2 * split * rest <= slots && k_pad / (2 * split) >= 4 * kChunkK) split *= 2;
+  return split;
+}
+
 // launch_tc_planes for a split_k = 1 configuration whose grid ends in a
 // partial wave: the whole waves of row tiles run as configured and the rows
-// of the last wave, when it would leave at least half of the SMs idle, run
-// as a second grid with K split across the idle SMs (disjoint rows of C, so
-// the results are those of split_k = 2..8 on those rows).  One CTA per SM:
-// M = 65536, N = 32 is 3 full waves of 148 tiles and 68 more.
+// of a last wave that tail_split splits as a second grid (disjoint rows of C,
+// so the results are those of split_k = 2..8 on those rows).
 template <int BN, int NS, int AM>
 hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
                            const __nv_bfloat16 *planes, int k_pad, int n_pad, int *err,
@@ -1126,11 +1356,7 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
   const int64_t tiles = (static_cast<int64_t>(p.M) + kBM - 1) / kBM;
   const int64_t slots = sm_count();
   const int64_t full = (tiles / slots) * slots;
-  const int64_t rest = tiles - full;
-  if (c.split_k != 1 || n_pad != BN || full == 0 || rest == 0 || 2 * rest > slots)
-    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, err, s);
-  int split = 1;
-  while (split < 8 && 2 * split * rest <= slots && k_pad / (2 * split) >= 4 * kChunkK) split *= 2;
+  const int split = c.split_k == 1 && n_pad == BN ? tail_split(tiles, slots, k_pad) : 1;
   if (split == 1) return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, err, s);
   const int64_t m1 = full * kBM;
   GemmProblem head = p, tail = p;
@@ -1143,6 +1369,33 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
   hml_status st = launch_tc_planes<BN, NS, AM>(head, c, planes, k_pad, n_pad, err, s);
   if (st != HML_STATUS_SUCCESS) return st;
   return launch_tc_planes<BN, NS, AM>(tail, ct, planes, k_pad, n_pad, err, s);
+}
+
+// The persistent form's work for a split_k = 1 configuration on the automatic
+// path; false where the grids above are as fast.  From two whole waves on it
+// saves their set-up and drain (B200: 65536 x 32 x 128 37.2 -> 27.9 us,
+// 60000 x 20 x 2047 136 -> 121, 65536 x 32 x 4096 216 -> 207, x 128 368 -> 364),
+// and from one wave on when the split tail occupies half of the SMs (28416 x
+// 32 x 1504 51.5 -> 48.5; a smaller tail's sum through memory costs what is
+// saved, 19200 x 128 x 4096 113 -> 116).  Several column tiles at a large K
+// stay with the grids: 8192^3 6.45 ms against 6.70 (4096^3 and 8192 x 4096 x
+// 8192 the same either way, 8192 x 2048 x 512 126 -> 111 us).
+bool tc_walk(const GemmProblem &p, const hml_sgemm_config &c, int bn, int k_pad, int n_pad,
+             TcWalk *w) {
+  const int64_t tiles =
+      (static_cast<int64_t>(p.M) + kBM - 1) / kBM * static_cast<int64_t>(n_pad / bn);
+  const int64_t slots = sm_count();
+  const int64_t full = tiles / slots * slots;
+  if (c.split_k != 1 || full == 0 || tiles == slots) return false;
+  if (n_pad != bn && p.K > 4096) return false;
+  w->whole = tiles;
+  const int split = n_pad == bn ? tail_split(tiles, slots, k_pad) : 1;
+  if (split > 1) {
+    w->whole = full;
+    w->tail = static_cast<int>(tiles - full);
+    w->tsplit = split;
+  }
+  return full > slots || 2 * static_cast<int64_t>(w->tail) * split > slots;
 }
 
 // B -> BF16 planes in `planes` ([NS][n_pad][k_pad]).
@@ -1184,10 +1437,20 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
   // B planes in the stream's workspace (FP16X3: then the column exponents)
   const size_t plane_bytes = static_cast<size_t>(n_pad) * k_pad * 2;
   const size_t planes_total = tc_geom(NS) * plane_bytes;
-  const size_t extra = NS == 5 ? static_cast<size_t>(n_pad) * sizeof(int) : 0;
+  size_t extra = NS == 5 ? static_cast<size_t>(n_pad) * sizeof(int) : 0;
+  TcWalk walk;
+  const bool persist = waves && NS <= 3 && tc_walk(p, c, BN, k_pad, n_pad, &walk);
+  if (persist)
+    extra = static_cast<size_t>(walk.tail) * walk.tsplit * BN * kBM * sizeof(float);
   void *ws = nullptr;
   hml_status st = workspace(planes_total + extra, s, &ws);
   if (st != HML_STATUS_SUCCESS) return st;
+  if (persist && walk.tail > 0) {
+    // planes_total is a multiple of 128 bytes (k_pad a multiple of 64)
+    walk.partial = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + planes_total);
+    st = tile_counters(static_cast<size_t>(walk.tail), s, &walk.arrivals);
+    if (st != HML_STATUS_SUCCESS) return st;
+  }
   auto *planes = static_cast<__nv_bfloat16 *>(ws);
   if constexpr (NS == 5) {
     // planes_total is a multiple of 128 bytes (k_pad a multiple of 64)
@@ -1199,6 +1462,11 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
   } else {
     st = split_b<NS>(p, planes, k_pad, n_pad, s);
     if (st != HML_STATUS_SUCCESS) return st;
+    if constexpr (NS <= 3) {
+      if (persist)
+        return launch_tc_planes<BN, NS, AM, true>(p, c, planes, k_pad, n_pad,
+                                                  device_error_word(), s, nullptr, &walk);
+    }
     if (waves)
       return launch_tc_waves<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s);
     return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s);
@@ -1671,7 +1939,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       tc_fence_after();
       const uint32_t dst = tA + lanes + static_cast<uint32_t>(o * SC);
       tmem_st16(dst, wv);
-      __syncwarp();  // every lane's values are in: see the single-problem kernel
+      __syncwarp();  // every lane's values are in: see release_early
       if (lane == 0) mbar_arrive(&aempty[s]);
       split_plane32<NS == 2>(x, wv);
       tmem_st16(dst + 16u, wv);

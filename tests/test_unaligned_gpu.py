@@ -64,7 +64,8 @@ def test_unaligned_tiles(cuda, ta, M, N, K):
 
 
 @pytest.mark.parametrize("ta", [0, 1])
-@pytest.mark.parametrize("M,N,K", [(3001, 45, 701), (517, 20, 9001)])  # whole K, split K
+# whole K, split K, several waves of tiles
+@pytest.mark.parametrize("M,N,K", [(3001, 45, 701), (517, 20, 9001), (40001, 20, 301)])
 def test_unaligned_not_finite(cuda, ta, M, N, K):
     """Infinities, NaN and the largest finite values give what plain FP32
     products give (their BF16 residuals alone would give NaN)."""
