@@ -15,6 +15,7 @@ hml_status fill_random(float *out, size_t n, uint64_t seed, uint64_t stream_id, 
                        cudaStream_t s);
 hml_status sgemm_error_fp64(const GemmProblem &p, const float *C0, double err[4], cudaStream_t s);
 hml_status release_all();
+void release_host_staging();
 int simt_num_shapes();
 void simt_shape(int v, int *bm, int *bn, int *wk);
 int tc_num_shapes();
@@ -397,7 +398,10 @@ hml_status hml_check_wait_limit(void *stream) {
   return check_wait_limit(static_cast<cudaStream_t>(stream));
 }
 
-hml_status hml_release_resources(void) { return release_all(); }
+hml_status hml_release_resources(void) {
+  release_host_staging();
+  return release_all();
+}
 
 uint64_t hml_launch_count(void) { return launch_count(); }
 
