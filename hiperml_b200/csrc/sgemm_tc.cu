@@ -1627,6 +1627,7 @@ struct TcBatchArgs {
   int nitems;
   unsigned *queue;              // [2]: queue head, CTAs finished (zero between launches)
   int sa, so;
+  int first;                    // the plan's first tile kernel
   int *err;
 };
 
@@ -1698,7 +1699,14 @@ __host__ __device__ constexpr int tcb_warps(int bn, int ns) {
 
 template <int BN, int NS>
 __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcBatchArgs args) {
-  allow_dependent_launch();  // the next tile kernel may take SMs this one leaves
+  // The tile kernels of a plan run at the same time: each is a programmatic
+  // dependent of the one before it, and its CTAs take the SMs that one
+  // leaves.  The first waits for the B planes (its B loader, the others start
+  // on A) and only then lets the second start, so a later kernel finds the
+  // planes complete and starts at once; its last CTA out waits for the kernel
+  // before it, so the last kernel ends when all have.  (One after another:
+  // 12 uneven problems 222 us, 134 like this; 60 problems 282, 265.)
+  if (!args.first) allow_dependent_launch();
   constexpr int G = tc_groups();
   constexpr int D = tcb_drain_groups(BN);
   constexpr int DC = BN / D;
@@ -1835,11 +1843,10 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
   } else if (warp == 1) {
     // -------------------------------------------------------- TMA, B
     if (lane == 0) {
-      // launched as a programmatic dependent of the previous kernel of the
-      // plan: the B planes are complete once that kernel is (the kernel
-      // before a tile kernel is the splitting kernel or another tile
-      // kernel, itself complete only after the splitting kernel)
-      wait_prior_grid();
+      if (args.first) {
+        wait_prior_grid();  // the splitting kernel
+        allow_dependent_launch();
+      }
       QueueCursor cur;
       bool ok = cur.fetch(args, ifull, iempty, iring, false, lane);
       for (int blk = 0; ok && !cur.end;) {
@@ -1991,16 +1998,23 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       if (lane == 0) mbar_arrive(&accempty[b]);
       if (cur.c == cur.it.cpt() - 1) {
         // the item's last chunk: C tile (row m, columns d*DC ..) and reset
-        const TcBatchProblem &pr = *cur.pr;
+        // (the record by value: read through the pointer it would be loaded
+        // again after every store, which cost 128-wide tiles 6 us each: 606208
+        // x 128 x 128 319 us, 167 like this; 60 uneven problems 265 -> 257)
+        const TcBatchProblem pr = *cur.pr;
         const int64_t gm = static_cast<int64_t>(cur.it.tm) * kBM + m;
         const int nb = cur.it.tn * BN + d * DC;
-        if (gm < pr.M) {
+        if (gm < pr.M && nb < pr.N) {
+          const int cols = min(DC, pr.N - nb);
+          float *cp = pr.C + gm * pr.scm + static_cast<int64_t>(nb) * pr.scn;
+          if (pr.beta == 0.0f) {
 #pragma unroll
-          for (int i = 0; i < DC; ++i) {
-            if (nb + i < pr.N) {
-              float *cp = pr.C + gm * pr.scm + static_cast<int64_t>(nb + i) * pr.scn;
-              *cp = axpby(pr.alpha, sums[i], pr.beta, cp);
-            }
+            for (int i = 0; i < DC; ++i, cp += pr.scn)
+              if (i < cols) *cp = axpby(pr.alpha, sums[i], 0.0f, cp);
+          } else {
+#pragma unroll
+            for (int i = 0; i < DC; ++i, cp += pr.scn)
+              if (i < cols) *cp = axpby(pr.alpha, sums[i], pr.beta, cp);
           }
         }
 #pragma unroll
@@ -2027,6 +2041,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       args.queue[0] = 0u;
       args.queue[1] = 0u;
       __threadfence();
+      if (!args.first) wait_prior_grid();
     }
   }
 }
@@ -2274,6 +2289,11 @@ hml_status tc_batch_create(const GemmProblem *probs, int count, cudaStream_t str
     tc_batch_destroy(b);
     return st;
   }
+  for (int c = 2; c >= 0; --c) {  // in launch order
+    if (b->cls[c].grid == 0) continue;
+    b->cls[c].args.first = 1;
+    break;
+  }
   b->nprob = count;
   b->items = static_cast<int>(total_items);
   b->splits = reinterpret_cast<const TcSplitDesc *>(base + o_split);
@@ -2289,10 +2309,8 @@ hml_status tc_batch_launch(const TcBatch *b, cudaStream_t s) {
       <<<dim3(static_cast<unsigned>(b->split_blocks), static_cast<unsigned>(b->nprob)), 256, 0,
          s>>>(b->splits);
   cudaError_t e = cudaGetLastError();
-  // each tile kernel is a programmatic dependent of the kernel before it:
-  // its CTAs start on the SMs that kernel has finished with, and only its B
-  // loader waits for that kernel to complete
-  // (the widest class, whose tiles take longest, first)
+  // each tile kernel is a programmatic dependent of the kernel before it (see
+  // the kernel's head); the widest class, whose tiles take longest, first
   for (int c = 2; c >= 0 && e == cudaSuccess; --c) {
     const TcBatch::Class &k = b->cls[c];
     if (k.grid == 0) continue;
