@@ -598,9 +598,11 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         sg->kbeg = sg->rank * args.tkc;
         sg->kend = min(p.K, sg->kbeg + args.tkc);
       }
-      const int64_t tiles_m = (static_cast<int64_t>(p.M) + kBM - 1) / kBM;
-      sg->m0 = t % tiles_m * kBM;
-      sg->n0 = static_cast<int>(t / tiles_m) * BN;
+      // (a 32-bit division: C's tiles are far fewer than 2^31)
+      const unsigned tiles_m = (static_cast<unsigned>(p.M) + kBM - 1) / kBM;
+      const unsigned tu = static_cast<unsigned>(t);
+      sg->m0 = static_cast<int64_t>(tu % tiles_m) * kBM;
+      sg->n0 = static_cast<int>(tu / tiles_m) * BN;
       sg->nkb = sg->kend > sg->kbeg ? (sg->kend - sg->kbeg + P * kBK - 1) / (P * kBK) * P : 0;
       return true;
     }
