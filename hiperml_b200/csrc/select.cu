@@ -152,9 +152,43 @@ bool v1_rule_config(const GemmProblem &p, int K_row, int N_row, hml_sgemm_config
   return true;
 }
 
+// A predicted split-BF16 configuration brought to the tile that holds N where
+// that is always the better one; the network, smooth in N and M, misses it
+// near the edges (65536 x 64 x 4096, A K-contiguous: 311 us with the 128-wide
+// tile it takes, 238; 14031 x 80 x 1488: 50 us with 64-wide ones, 36).  Over
+// 5000 measured shapes:
+//   * a tile twice as wide as N needs was at best 1.4 % faster (288 shapes with
+//     32 < N <= 64; at the median 15 % slower; narrower N likewise);
+//   * several narrower tiles were not faster by 3 % in any of 251 shapes whose
+//     row tiles fill more than half of the SMs but one wave, or two waves and
+//     more (at the median 20 to 40 % slower; elsewhere they often win);
+//   * from two waves on, K was better whole in all of 141 shapes;
+//   * SIMT tiles narrower than 9 <= N <= 128, which read A several times, were
+//     slower in all of 217 shapes with K >= 300 and more than half a wave of
+//     row tiles (21591 x 9 x 3392 row-major: 298 us, 64).
+static void fit_tile_to_n(const GemmProblem &p, hml_sgemm_config *c) {
+  const int64_t tiles = (static_cast<int64_t>(p.M) + 127) / 128, sms = sm_count();
+  const bool reread = c->algo == HML_ALGO_SIMT && c->tile_n < p.N && p.N > 8 && p.K >= 300 &&
+                      2 * tiles > sms;
+  if (!reread && c->algo != HML_ALGO_BF16X6 && c->algo != HML_ALGO_BF16X3) return;
+  const int algo = reread ? static_cast<int>(HML_ALGO_BF16X6) : c->algo;
+  hml_sgemm_config n = heuristic_config(p, algo);
+  if (n.algo != algo) return;
+  const bool holds = n.tile_n >= p.N;
+  const bool waves = tiles >= 2 * sms, one = 2 * tiles > sms && tiles <= sms;
+  const bool wider = !reread && 2 * n.tile_n <= c->tile_n;
+  const bool narrower = holds && c->tile_n < n.tile_n && (reread || waves || one);
+  if (!wider && !narrower && !(holds && waves && !reread && c->split_k > 1)) return;
+  n.split_k = waves || narrower ? 1 : c->split_k;
+  if (check_config_ok(p, n)) *c = n;
+}
+
 hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s) {
   if (tuned_lookup(p, c) && check_config_ok(p, *c)) return HML_STATUS_SUCCESS;
-  if (predictor_lookup(p, c, s) && check_config_ok(p, *c)) return HML_STATUS_SUCCESS;
+  if (predictor_lookup(p, c, s) && check_config_ok(p, *c)) {
+    fit_tile_to_n(p, c);
+    return HML_STATUS_SUCCESS;
+  }
   // Measured on B200 (M = 65536, K = 4096): FP32 SIMT wins at N <= 16 (the
   // HBM-bound GEMV-like shapes); the split-BF16 tensor-core forms win from
   // N = 32 on.  BF16X6 keeps FP32-level accuracy; BF16X3 (faster, ~2**-17)
@@ -172,12 +206,14 @@ hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t
 }
 
 // Where the tensor cores take a problem whose A TMA cannot address as it
-// stands: wherever they would take it with an addressable A, and from
-// M K max(N, 8) = 2^25 on also where SIMT would.  The SIMT tiles then stage A
-// with 4-byte cp.async and fall behind early (B200, odd K row-major: 2048 x
-// 16 x 1025, at the line, 16.9 us against 16.4; 8192 x 4 x 1025 26.6 against
-// 25.2; 32768 x 8 x 1025 82 against 48; 32768 x 64 x 3001 737 against 119);
-// below it one launch beats two (2048 x 8 x 257 13.2 us against 16.5).
+// stands: wherever they would take it with an addressable A, and where SIMT
+// would from M K max(N, 8) = 2^25 on, with 40 row tiles from M K N = 2^24 on.
+// The SIMT tiles then stage A with 4-byte cp.async and fall behind early
+// (B200, odd K row-major: 2048 x 16 x 1025, at the line, 15.0 us against 12.1;
+// 32768 x 8 x 1025 82 against 48; 32768 x 64 x 3001 737 against 119; 5968 x 10
+// x 438 18.9 against 12.6; 12001 x 6 x 301 15.5 against 11.1); below the lines
+// one launch beats two (2048 x 8 x 257 7.8 us against 10.3; 4001 x 12 x 501
+// 12.7 against 14.1; 30001 x 2 x 101 10.8 against 13.3).
 bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s) {
   const int64_t ld = p.a_kcontig() ? p.sam : p.sak;
   const bool base_ok = (reinterpret_cast<uintptr_t>(p.A) & 15u) == 0;
@@ -188,8 +224,10 @@ bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s)
   (p.a_kcontig() ? q.sam : q.sak) = (ld + 3) / 4 * 4;
   if (select_config(q, c, s) != HML_STATUS_SUCCESS) return false;
   if (c->algo == HML_ALGO_BF16X6) return true;
-  const double work = static_cast<double>(p.M) * p.K * std::max(p.N, 8);
-  if (c->algo == HML_ALGO_SIMT && work < 0x1p25) return false;
+  const double mk = static_cast<double>(p.M) * p.K;
+  if (c->algo == HML_ALGO_SIMT && mk * std::max(p.N, 8) < 0x1p25 &&
+      (p.M < 40 * 128 || mk * p.N < 0x1p24))
+    return false;
   *c = heuristic_config(q, HML_ALGO_BF16X6);
   return true;
 }
