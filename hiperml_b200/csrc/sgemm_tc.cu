@@ -1381,13 +1381,14 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
 
 // The persistent form's work for a split_k = 1 configuration on the automatic
 // path; false where the grids above are as fast.  From two whole waves on it
-// saves their set-up and drain (B200: 65536 x 32 x 128 37.2 -> 27.9 us,
-// 60000 x 20 x 2047 136 -> 121, 65536 x 32 x 4096 216 -> 207, x 128 368 -> 364),
-// and from one wave on when the split tail occupies half of the SMs (28416 x
-// 32 x 1504 51.5 -> 48.5; a smaller tail's sum through memory costs what is
-// saved, 19200 x 128 x 4096 113 -> 116).  Several column tiles at a large K
-// stay with the grids: 8192^3 6.45 ms against 6.70 (4096^3 and 8192 x 4096 x
-// 8192 the same either way, 8192 x 2048 x 512 126 -> 111 us).
+// saves their set-up and drain (B200, grids -> persistent: 40000 x 64 x 200
+// 26.3 -> 20.9 us, 37888 x 32 x 512 25.0 -> 21.7, 56832 x 16 x 1000 58.8 ->
+// 50.1, 65536 x 128 x 1024 109 -> 96, 65536 x 32 x 4096 216 -> 209), and from
+// one wave on when the split tail occupies half of the SMs (28416 x 32 x 1504
+// 45.3 -> 43.3; a smaller tail's sum through memory costs what is saved:
+// 21001 x 100 x 501 35.4 -> 37.4, 19200 x 128 x 4096 115 -> 112).  Several
+// column tiles at a large K stay with the grids: 8192^3 6.45 ms against 6.70
+// (8192 x 4096 x 2048 825 -> 721 us).
 bool tc_walk(const GemmProblem &p, const hml_sgemm_config &c, int bn, int k_pad, int n_pad,
              TcWalk *w) {
   const int64_t tiles =
