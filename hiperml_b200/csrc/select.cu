@@ -155,30 +155,27 @@ bool v1_rule_config(const GemmProblem &p, int K_row, int N_row, hml_sgemm_config
 // A predicted split-BF16 configuration brought to the tile that holds N where
 // that is always the better one; the network, smooth in N and M, misses it
 // near the edges (65536 x 64 x 4096, A K-contiguous: 311 us with the 128-wide
-// tile it takes, 238; 14031 x 80 x 1488: 50 us with 64-wide ones, 36).  Over
+// tile it takes, 238 with the 64-wide; 14031 x 80 x 1488: 36 us with the
+// 128-wide, 50 with two 64-wide).  Over
 // 5000 measured shapes:
 //   * a tile twice as wide as N needs was at best 1.4 % faster (288 shapes with
 //     32 < N <= 64; at the median 15 % slower; narrower N likewise);
 //   * several narrower tiles were not faster by 3 % in any of 251 shapes whose
 //     row tiles fill more than half of the SMs but one wave, or two waves and
 //     more (at the median 20 to 40 % slower; elsewhere they often win);
-//   * from two waves on, K was better whole in all of 141 shapes;
-//   * SIMT tiles narrower than 9 <= N <= 128, which read A several times, were
-//     slower in all of 217 shapes with K >= 300 and more than half a wave of
-//     row tiles (21591 x 9 x 3392 row-major: 298 us, 64).
+//   * from two waves on, K was better whole in all of 141 shapes.
+// The family stays the network's: the SIMT sums of a short K are closer to the
+// exact ones (about 1e-7 of the largest, BF16X6 5e-7).
 static void fit_tile_to_n(const GemmProblem &p, hml_sgemm_config *c) {
+  if (c->algo != HML_ALGO_BF16X6 && c->algo != HML_ALGO_BF16X3) return;
+  hml_sgemm_config n = heuristic_config(p, c->algo);
+  if (n.algo != c->algo) return;
   const int64_t tiles = (static_cast<int64_t>(p.M) + 127) / 128, sms = sm_count();
-  const bool reread = c->algo == HML_ALGO_SIMT && c->tile_n < p.N && p.N > 8 && p.K >= 300 &&
-                      2 * tiles > sms;
-  if (!reread && c->algo != HML_ALGO_BF16X6 && c->algo != HML_ALGO_BF16X3) return;
-  const int algo = reread ? static_cast<int>(HML_ALGO_BF16X6) : c->algo;
-  hml_sgemm_config n = heuristic_config(p, algo);
-  if (n.algo != algo) return;
   const bool holds = n.tile_n >= p.N;
   const bool waves = tiles >= 2 * sms, one = 2 * tiles > sms && tiles <= sms;
-  const bool wider = !reread && 2 * n.tile_n <= c->tile_n;
-  const bool narrower = holds && c->tile_n < n.tile_n && (reread || waves || one);
-  if (!wider && !narrower && !(holds && waves && !reread && c->split_k > 1)) return;
+  const bool wider = 2 * n.tile_n <= c->tile_n;
+  const bool narrower = holds && c->tile_n < n.tile_n && (waves || one);
+  if (!wider && !narrower && !(holds && waves && c->split_k > 1)) return;
   n.split_k = waves || narrower ? 1 : c->split_k;
   if (check_config_ok(p, n)) *c = n;
 }
@@ -213,7 +210,10 @@ hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t
 // 32768 x 8 x 1025 82 against 48; 32768 x 64 x 3001 737 against 119; 5968 x 10
 // x 438 18.9 against 12.6; 12001 x 6 x 301 15.5 against 11.1); below the lines
 // one launch beats two (2048 x 8 x 257 7.8 us against 10.3; 4001 x 12 x 501
-// 12.7 against 14.1; 30001 x 2 x 101 10.8 against 13.3).
+// 12.7 against 14.1; 30001 x 2 x 101 10.8 against 13.3).  Not below K = 100:
+// from there on the error is no larger than SIMT's (RMS 0.7 to 0.9 of it over
+// N = 2 to 100, K = 101 to 3001), at K = 65 its maximum is (1.7e-7 against
+// 1.2e-7).
 bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s) {
   const int64_t ld = p.a_kcontig() ? p.sam : p.sak;
   const bool base_ok = (reinterpret_cast<uintptr_t>(p.A) & 15u) == 0;
@@ -225,8 +225,8 @@ bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s)
   if (select_config(q, c, s) != HML_STATUS_SUCCESS) return false;
   if (c->algo == HML_ALGO_BF16X6) return true;
   const double mk = static_cast<double>(p.M) * p.K;
-  if (c->algo == HML_ALGO_SIMT && mk * std::max(p.N, 8) < 0x1p25 &&
-      (p.M < 40 * 128 || mk * p.N < 0x1p24))
+  if (c->algo == HML_ALGO_SIMT &&
+      (p.K < 100 || (mk * std::max(p.N, 8) < 0x1p25 && (p.M < 40 * 128 || mk * p.N < 0x1p24))))
     return false;
   *c = heuristic_config(q, HML_ALGO_BF16X6);
   return true;
