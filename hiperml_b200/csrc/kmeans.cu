@@ -38,6 +38,7 @@
 
 #include "hml_device.cuh"
 #include "hml_internal.h"
+#include "hml_lines.h"
 #include "hml_select.h"
 #include "hml_tune.h"
 #include "hml_tcgen05.cuh"
@@ -1347,11 +1348,10 @@ hml_status assign_tc_rows(const KmTcPlan &p, const float *points, int np, int d,
   memset(&tm, 0, sizeof tm);
   if constexpr (AU) {
     for (int r = 0; r < 4; ++r) {
-      const float *first = points + static_cast<int64_t>(r) * d;
-      a.e[r] = static_cast<int>((reinterpret_cast<uintptr_t>(first) & 15u) / 4);
-      if (!tensor_map_2d(&tm.m[r], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, first - a.e[r], d + a.e[r],
-                         (np - r + 3) / 4, static_cast<uint64_t>(d) * 16, 36, 32,
-                         CU_TENSOR_MAP_SWIZZLE_NONE))
+      const LineClass c4 = line_class(points, d, np, d, r);
+      a.e[r] = c4.skip;
+      if (!tensor_map_2d(&tm.m[r], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, c4.base, c4.len, c4.lines,
+                         c4.stride, 36, 32, CU_TENSOR_MAP_SWIZZLE_NONE))
         return HML_STATUS_CUDA_ERROR;
     }
   } else if (!tensor_map_2d(&tm.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, points, d, np,

@@ -132,9 +132,9 @@ bool tensor_map_2d(CUtensorMap *map, CUtensorMapDataType dtype, const void *base
     }
   }
   if (dim0 == 0 || dim1 == 0) {
-    // a zero extent is not encodable; such problems never launch a load
-    dim0 = dim0 ? dim0 : 1;
-    dim1 = dim1 ? dim1 : 1;
+    // not encodable, and rounded up it would let loads read what is not there
+    t_last_error = "tensor map of an empty matrix";
+    return false;
   }
   cuuint64_t dims[2] = {dim0, dim1};
   cuuint64_t strides[1] = {stride1_bytes};

@@ -56,6 +56,7 @@
 
 #include "hml_device.cuh"
 #include "hml_internal.h"
+#include "hml_lines.h"
 #include "hml_tcgen05.cuh"
 
 namespace hml {
@@ -1256,18 +1257,12 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   TcArgs args = {};
   bool ok = true;
   if constexpr (am_unaligned(AM)) {
-    // lines 4 j + r of A (M and K are at least 4): each class from the
-    // 16-byte boundary at or before its first line, whose granule the
-    // line's first float shares
     const bool ak = AM == kAKU;
-    const int64_t ld = ak ? p.sam : p.sak;
-    const int lines = ak ? p.M : p.K, len = ak ? p.K : p.M;
     for (int r = 0; r < 4 && ok; ++r) {
-      const float *first = p.A + r * ld;
-      args.e[r] = static_cast<int>((reinterpret_cast<uintptr_t>(first) & 15u) / 4);
-      ok = tensor_map_2d(&ta.m[r], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, first - args.e[r],
-                         len + args.e[r], (lines - r + 3) / 4, ld * 16, ak ? 36 : 132,
-                         ak ? 32 : 8, CU_TENSOR_MAP_SWIZZLE_NONE);
+      const LineClass c4 = line_class(p.A, ak ? p.sam : p.sak, ak ? p.M : p.K, ak ? p.K : p.M, r);
+      args.e[r] = c4.skip;
+      ok = tensor_map_2d(&ta.m[r], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, c4.base, c4.len, c4.lines,
+                         c4.stride, ak ? 36 : 132, ak ? 32 : 8, CU_TENSOR_MAP_SWIZZLE_NONE);
     }
   } else if (AM == kAK)
     ok = tensor_map_2d(&ta.m[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.A, p.K, p.M, p.sam * 4, kBK,
