@@ -117,9 +117,16 @@ int *device_error_word_if_any();  // nullptr when not allocated yet (allocates n
 // Reads and clears the allocation-free entry point's error word (sgemm_tc.cu).
 hml_status noalloc_take_error(int *code);
 hml_status workspace(size_t bytes, cudaStream_t s, void **ptr);
-// The same for a second, independent buffer per (device, stream): slot 1 holds
-// data that outlives a library call made in between (which uses slot 0).
+// The same for independent buffers per (device, stream): slot 1 holds data that
+// outlives a library call made in between (which uses slot 0), slot 2 the
+// persistent split-BF16 kernel's tail sums, of one size for every problem.
+constexpr int kWorkspaceSlots = 3;
 hml_status workspace_slot(int slot, size_t bytes, cudaStream_t s, void **ptr);
+// Whether a request would be met without an allocation, which a stream under
+// capture may not be able to make.
+bool workspace_held(int slot, size_t bytes, cudaStream_t s);
+bool tile_counters_held(size_t n, cudaStream_t s);
+bool stream_capturing(cudaStream_t s);
 // n zero-initialised counters private to (device, stream).  Kernels that use
 // them leave every counter at zero again when they finish.
 hml_status tile_counters(size_t n, cudaStream_t s, unsigned **ptr);

@@ -20,8 +20,7 @@ struct Ws {
   void *ptr = nullptr;
   size_t bytes = 0;
 };
-std::map<std::pair<int, cudaStream_t>, Ws> g_ws;
-std::map<std::pair<int, cudaStream_t>, Ws> g_ws1;  // a second buffer per stream (slot 1)
+std::map<std::pair<int, cudaStream_t>, Ws> g_ws[kWorkspaceSlots];
 std::map<std::pair<int, cudaStream_t>, Ws> g_counters;
 std::map<int, int> g_sms;
 thread_local std::string t_last_error;
@@ -92,7 +91,7 @@ hml_status workspace(size_t bytes, cudaStream_t s, void **ptr) { return workspac
 hml_status workspace_slot(int slot, size_t bytes, cudaStream_t s, void **ptr) {
   const int d = current_device();
   std::lock_guard<std::mutex> lk(g_mu);
-  Ws &w = (slot == 0 ? g_ws : g_ws1)[std::make_pair(d, s)];
+  Ws &w = g_ws[slot][std::make_pair(d, s)];
   if (w.bytes < bytes) {
     if (w.ptr) {
       // earlier work on this stream may still use the old buffer
@@ -112,6 +111,29 @@ hml_status workspace_slot(int slot, size_t bytes, cudaStream_t s, void **ptr) {
   }
   *ptr = w.ptr;
   return HML_STATUS_SUCCESS;
+}
+
+bool workspace_held(int slot, size_t bytes, cudaStream_t s) {
+  const int d = current_device();
+  std::lock_guard<std::mutex> lk(g_mu);
+  auto it = g_ws[slot].find(std::make_pair(d, s));
+  return it != g_ws[slot].end() && it->second.bytes >= bytes;
+}
+
+bool tile_counters_held(size_t n, cudaStream_t s) {
+  const int d = current_device();
+  std::lock_guard<std::mutex> lk(g_mu);
+  auto it = g_counters.find(std::make_pair(d, s));
+  return it != g_counters.end() && it->second.bytes >= n * sizeof(unsigned);
+}
+
+bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while another one is captured
+    return true;
+  }
+  return cs != cudaStreamCaptureStatusNone;
 }
 
 bool tensor_map_2d(CUtensorMap *map, CUtensorMapDataType dtype, const void *base, uint64_t dim0,
@@ -182,12 +204,11 @@ hml_status tile_counters(size_t n, cudaStream_t s, unsigned **ptr) {
 hml_status release_all() {
   std::lock_guard<std::mutex> lk(g_mu);
   cudaDeviceSynchronize();
-  for (auto &kv : g_ws)
-    if (kv.second.ptr) cudaFree(kv.second.ptr);
-  g_ws.clear();
-  for (auto &kv : g_ws1)
-    if (kv.second.ptr) cudaFree(kv.second.ptr);
-  g_ws1.clear();
+  for (auto &slot : g_ws) {
+    for (auto &kv : slot)
+      if (kv.second.ptr) cudaFree(kv.second.ptr);
+    slot.clear();
+  }
   for (auto &kv : g_counters)
     if (kv.second.ptr) cudaFree(kv.second.ptr);
   g_counters.clear();

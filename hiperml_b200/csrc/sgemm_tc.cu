@@ -1235,7 +1235,6 @@ bool tc_config_fits(int bn, int ns, int stages) {
 
 namespace {
 
-// Launch of the kernel with the B planes already split into `planes`.
 // The persistent form's work: see TcArgs.
 struct TcWalk {
   int64_t whole = 0;
@@ -1244,6 +1243,7 @@ struct TcWalk {
   unsigned *arrivals = nullptr;
 };
 
+// Launch of the kernel with the B planes already split into `planes`.
 template <int BN, int NS, int AM, bool PERSIST = false>
 hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
                             const __nv_bfloat16 *planes, int k_pad, int n_pad, int *err,
@@ -1402,6 +1402,29 @@ bool tc_walk(const GemmProblem &p, const hml_sgemm_config &c, int bn, int k_pad,
   return full > slots || 2 * static_cast<int64_t>(w->tail) * split > slots;
 }
 
+// The tail's partial sums and counters.  A problem's own need follows M modulo
+// the rows of a wave, so that a smaller problem can need more than a larger one
+// and would grow a buffer that a graph captured before it uses; the stream's
+// first tensor-core call on the automatic path therefore reserves what any
+// problem's tail can take (a CTA's tile each: tail * tsplit <= SMs, 9.7 MB on
+// 148).  False when that is not to be had, under capture by a stream that did
+// not make such a call: the tail then runs as a grid, with the same bits.
+bool tail_buffers(cudaStream_t s, TcWalk *w) {
+  const size_t sms = static_cast<size_t>(sm_count());
+  const size_t bytes = sms * kTcShapes[kNumTcShapes - 1].bn * kBM * sizeof(float);
+  const bool held = workspace_held(2, bytes, s) && tile_counters_held(sms, s);
+  if (held && w->tail == 0) return true;
+  if (!held && stream_capturing(s)) return false;
+  void *ws = nullptr;
+  if (workspace_slot(2, bytes, s, &ws) != HML_STATUS_SUCCESS ||
+      tile_counters(sms, s, &w->arrivals) != HML_STATUS_SUCCESS) {
+    cudaGetLastError();
+    return false;
+  }
+  w->partial = static_cast<float *>(ws);
+  return true;
+}
+
 // B -> BF16 planes in `planes` ([NS][n_pad][k_pad]).
 template <int NS>
 hml_status split_b(const GemmProblem &p, __nv_bfloat16 *planes, int k_pad, int n_pad,
@@ -1441,19 +1464,15 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
   // B planes in the stream's workspace (FP16X3: then the column exponents)
   const size_t plane_bytes = static_cast<size_t>(n_pad) * k_pad * 2;
   const size_t planes_total = tc_geom(NS) * plane_bytes;
-  size_t extra = NS == 5 ? static_cast<size_t>(n_pad) * sizeof(int) : 0;
-  TcWalk walk;
-  const bool persist = waves && NS <= 3 && tc_walk(p, c, BN, k_pad, n_pad, &walk);
-  if (persist)
-    extra = static_cast<size_t>(walk.tail) * walk.tsplit * BN * kBM * sizeof(float);
+  const size_t extra = NS == 5 ? static_cast<size_t>(n_pad) * sizeof(int) : 0;
   void *ws = nullptr;
   hml_status st = workspace(planes_total + extra, s, &ws);
   if (st != HML_STATUS_SUCCESS) return st;
-  if (persist && walk.tail > 0) {
-    // planes_total is a multiple of 128 bytes (k_pad a multiple of 64)
-    walk.partial = reinterpret_cast<float *>(static_cast<uint8_t *>(ws) + planes_total);
-    st = tile_counters(static_cast<size_t>(walk.tail), s, &walk.arrivals);
-    if (st != HML_STATUS_SUCCESS) return st;
+  TcWalk walk;
+  bool persist = false;
+  if constexpr (NS <= 3) {
+    persist = waves && tc_walk(p, c, BN, k_pad, n_pad, &walk);
+    if (waves && !tail_buffers(s, &walk) && walk.tail > 0) persist = false;
   }
   auto *planes = static_cast<__nv_bfloat16 *>(ws);
   if constexpr (NS == 5) {
