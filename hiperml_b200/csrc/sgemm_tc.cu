@@ -1465,6 +1465,9 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
   const size_t plane_bytes = static_cast<size_t>(n_pad) * k_pad * 2;
   const size_t planes_total = tc_geom(NS) * plane_bytes;
   const size_t extra = NS == 5 ? static_cast<size_t>(n_pad) * sizeof(int) : 0;
+  // (an unaligned A has the SIMT tiles, which need none, to fall back on)
+  if (am_unaligned(AM) && !workspace_held(0, planes_total + extra, s) && stream_capturing(s))
+    return HML_STATUS_ALLOC_FAILED;
   void *ws = nullptr;
   hml_status st = workspace(planes_total + extra, s, &ws);
   if (st != HML_STATUS_SUCCESS) return st;

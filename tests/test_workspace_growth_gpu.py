@@ -1,22 +1,25 @@
 """Workspaces of the tensor-core path and CUDA graphs (GPU): after one call of the
 largest shape on a stream, no smaller one may move a buffer that a captured
 graph uses or need an allocation inside a capture -- although a smaller problem
-can have a split last wave where the larger one has none.
+can have a split last wave where the larger one has none.  And a call on an A
+that TMA cannot address, which the SIMT tiles serve without a workspace, can be
+captured by a stream that made no call before.
 """
 import pytest
 
 import hiperml_b200 as hml
 from hiperml_b200._lib import lib
+from tests.gpu_util import gamma
 
 pytestmark = pytest.mark.gpu
 N, K = 32, 1024
 
 
-def operands(M, N, K):
+def operands(M, N, K, order="col"):
     import torch
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
-    A = torch.empty(K, M, device="cuda").uniform_(-1, 1, generator=g)
-    B = torch.empty(N, K, device="cuda").uniform_(-1, 1, generator=g)
+    A = torch.empty(*((K, M) if order == "col" else (M, K)), device="cuda").uniform_(-1, 1, generator=g)
+    B = torch.empty(*((N, K) if order == "col" else (K, N)), device="cuda").uniform_(-1, 1, generator=g)
     return A, B
 
 
@@ -113,4 +116,24 @@ def test_tail_without_its_buffer(sizes):
         assert torch.equal(c, want)
         s.synchronize()
         del g
+    assert hml.device_error() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(2049, 20, 1501), (20011, 45, 701)])
+def test_unaligned_call_captured_first(sizes, M, N, K):
+    import torch
+    A, B = operands(M, N, K, "row")
+    C = torch.zeros(M, N, device="cuda")
+    hml.sgemm(A, B)  # on another stream: the device's own set-up
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    lib.hml_release_resources()
+    with torch.cuda.stream(s):
+        g = capture(s, lambda: hml.sgemm_ex(1, 0, 0, M, N, K, 1.0, A, K, B, N, 0.0, C, N))
+        g.replay()
+        s.synchronize()
+        del g
+    exact = A.double() @ B.double()
+    bound = 2 * gamma(K + 2) * (A.double().abs() @ B.double().abs())
+    assert ((C.double() - exact).abs() <= bound).all()
     assert hml.device_error() == 0
