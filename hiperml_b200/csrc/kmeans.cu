@@ -87,7 +87,8 @@ __device__ __forceinline__ float ref_dist(const float *x, const float *c, int d)
 // the reference's own distance (sequential, subtract then FMA) and keeps the
 // first smallest below FLT_MAX (strict <), which is the reference's pick.
 // 0 when no candidate's distance is below FLT_MAX (the reference leaves that
-// case unset).
+// case unset).  A limit that is not finite (norms or products beyond FP32,
+// where g says nothing) makes every centroid a candidate.
 __device__ __noinline__ uint32_t exact_pick(const float *x, int d, const float *cent, int k,
                                             const float *cnorm, float lim) {
   constexpr int U = 16;  // centroids in flight: their loads and shuffle trees interleave
@@ -114,7 +115,7 @@ __device__ __noinline__ uint32_t exact_pick(const float *x, int d, const float *
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int c = c0 + u;
-      if (c >= k || !(fmaf(-2.0f, part[u], cnv[u]) <= lim)) continue;
+      if (c >= k || !(fmaf(-2.0f, part[u], cnv[u]) <= lim || !(lim < INFINITY))) continue;
       const float dist = ref_dist(x, cent + static_cast<int64_t>(c) * d, d);
       if (dist < bd) {
         bd = dist;
@@ -159,9 +160,11 @@ __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, cons
   int bk = -1;
   for (int c = lane; c < k; c += 32) {
     const float *cp = cs + c * st;
-    float dot = 0.0f;
-    for (int j = 0; j < d; ++j) dot = fmaf(xs[j], cp[j], dot);
-    if (!(fmaf(-2.0f, dot, cn[c]) <= lim)) continue;
+    if (lim < INFINITY) {
+      float dot = 0.0f;
+      for (int j = 0; j < d; ++j) dot = fmaf(xs[j], cp[j], dot);
+      if (!(fmaf(-2.0f, dot, cn[c]) <= lim)) continue;
+    }  // else: every centroid is a candidate (see exact_pick)
     const float dist = ref_dist(xs, cp, d);
     if (dist < bd) {
       bd = dist;
@@ -276,7 +279,7 @@ __global__ void kmeans_pick_kernel(const float *points, int64_t np, int d, int k
       lim = gmin + bound * (xn + cmax) + 1e-37f;
       int cand = 0;
       for (int c = 0; c < k; ++c) cand += fmaf(-2.0f, sp[c * lds], s_cnorm[c]) <= lim;
-      close = cand != 1;
+      close = cand != 1 || !(lim < INFINITY);
       if (!close) out[p] = static_cast<uint32_t>(kmin);
     }
     push_close(ccount, citems, p, lim, close);
@@ -1053,7 +1056,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       if (!ok) break;
       const int64_t p = (blockIdx.x + (g + static_cast<int64_t>(it) * W) * gridDim.x) * kTP + m;
       const bool live = p < a.np;
-      const float lim = g1 + margin;
+      const float lim = margin < INFINITY ? g1 + margin : INFINITY;
       close = live && (close || !(lim < INFINITY));
       if (live && !close) a.out[p] = static_cast<uint32_t>(k1);
       const unsigned vote = __ballot_sync(0xffffffffu, close);
