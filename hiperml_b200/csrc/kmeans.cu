@@ -13,7 +13,7 @@
 // centroid are one skinny GEMM S = X C^T (points x clusters), in one of three
 // forms:
 //   * tensor-core (method 3, the default wherever its kernel can run: at most
-//     256 centroids that fit in shared memory as BF16 planes): BF16X3 products
+//     256 centroids that fit in shared memory as FP16 planes): FP16X3 products
 //     on tcgen05 into TMEM, the argmin read back from the accumulator by the
 //     thread that owns the point;
 //   * tiled (method 1, the default otherwise up to 256 dimensions): a
@@ -24,13 +24,15 @@
 // The products carry rounding errors that the reference's direct sums do
 // not, so the pick is made exact: with g_k = ||c_k||^2 - 2 S_k, every
 // centroid whose g_k lies within a bound of the smallest (16 gamma_{dims+4}
-// (||x||^2 + max_k ||c_k||^2) for the FP32 forms, 2^-15 of it more for the
-// BF16X3 products: more than twice the sum of the worst-case errors of g and
+// (||x||^2 + max_k ||c_k||^2) for the FP32 forms, 2^-19 of it more for the
+// FP16X3 products: more than twice the sum of the worst-case errors of g and
 // of the reference's dist) is a candidate, and the reference's choice is
 // always among them.  A point with more than one candidate (or non-finite
 // values) goes to a close-call list that is settled with the reference's own
 // arithmetic over the candidates, the first smallest in increasing k.  So
 // every point gets the reference kernel's index, exact ties included.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
@@ -161,9 +163,13 @@ __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, cons
   for (int c = lane; c < k; c += 32) {
     const float *cp = cs + c * st;
     if (lim < INFINITY) {
-      float dot = 0.0f;
-      for (int j = 0; j < d; ++j) dot = fmaf(xs[j], cp[j], dot);
-      if (!(fmaf(-2.0f, dot, cn[c]) <= lim)) continue;
+      float dot[4] = {};
+      int j = 0;
+      for (; j + 4 <= d; j += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) dot[u] = fmaf(xs[j + u], cp[j + u], dot[u]);
+      for (; j < d; ++j) dot[0] = fmaf(xs[j], cp[j], dot[0]);
+      if (!(fmaf(-2.0f, (dot[0] + dot[1]) + (dot[2] + dot[3]), cn[c]) <= lim)) continue;
     }  // else: every centroid is a candidate (see exact_pick)
     const float dist = ref_dist(xs, cp, d);
     if (dist < bd) {
@@ -631,15 +637,21 @@ __global__ void __launch_bounds__(kTThreads, 2) kmeans_resident_kernel(
 // memory)  One persistent CTA per SM screens 128-point tiles on tcgen05 and
 // settles its own close calls; nothing runs before or after it.
 //
-// Products.  x = x0 + x1 and -2c = c0 + c1 in BF16 (16 significant bits each)
-// and -2 x.c ~ x0.c0 + x0.c1 + x1.c0 accumulated in FP32 in TMEM.  This only
-// screens: the split leaves out at most 3.02 2^-18 |x_j c_j| of a product (so
-// 3.02 2^-18 (||x||^2 + ||c||^2) of a g_k), and a point is settled from the
-// screen only when its second smallest g lies further from the smallest than
-// twice that and the FP32 margin together, 2^-15 + 16 gamma_{dims+4} times
-// ||x||^2 + max ||c||^2 (about the 32 gamma_{dims+4} that TF32X3 products were
-// given before; half their MMAs and half their TMEM).  Every other point gets
-// the reference's own FP32 arithmetic.
+// Products.  Points and centroids are scaled by one power of two s (exact)
+// that brings the largest coordinate of the centroids into [2^5, 2^6); then
+// x = x0 + x1 and -2c = c0 + c1 in FP16, 22 significant bits, and
+// -2 x.c ~ x0.c0 + x0.c1 + x1.c0 accumulated in FP32 in TMEM.  This only
+// screens.  The split leaves out at most 3.02 2^-22 |x_j 2 c_j| and, where a
+// half is subnormal, 1.01 2^-25 (|x_j| + |2 c_j|) of a product; with
+// max ||c|| >= 2^5 and dims <= 2048 that is at most 3.42 2^-22 (||x||^2 +
+// max ||c||^2) of a g_k, and a point is settled from the screen only when its
+// second smallest g lies further from the smallest than twice that and the
+// FP32 margin together, (2^-19 + 16 gamma_{dims+4}) (||x||^2 + max ||c||^2).
+// Every other point gets the reference's own FP32 arithmetic, and so does one
+// with ||x|| s >= 2^15.5, whose halves could overflow.
+// (BF16 halves need no scale and 16 packed instructions less a block, but a
+// margin of 2^-15: points far from the origin became close calls, 200k x 30,
+// k = 200 at an offset of 100 spreads 671 us.)
 //
 // Roles of a CTA (W = 4 or 2 groups, each with 512 / W TMEM columns: an
 // accumulator of NC columns, then S stages of 32 columns of A):
@@ -696,15 +708,24 @@ struct KmTcArgs {
 
 __host__ __device__ constexpr int km_tc_threads(int w) { return (4 + 4 * w) * 32; }
 
-__device__ __forceinline__ uint32_t km_bf16x2(float lo, float hi) {
+__device__ __forceinline__ uint32_t km_f16x2(float lo, float hi) {
   uint32_t r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
 
-// The values a packed BF16 pair holds.
-__device__ __forceinline__ float2 km_bf16_pair(uint32_t w) {
-  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+// The values a packed FP16 pair holds.
+__device__ __forceinline__ float2 km_f16_pair(uint32_t w) {
+  return __half22float2(*reinterpret_cast<const __half2 *>(&w));
+}
+
+// The power of two that brings magnitudes up to `top` (not NaN) below 2^6: at
+// most 2^105, so that 1 / s is normal (g of centroids that small all lie within
+// the margin's 1e-37), and 1 when there is nothing to scale.
+__device__ __forceinline__ float km_scale(float top) {
+  const int e = __float_as_int(top) >> 23;  // biased
+  if (top == 0.0f || e == 255) return 1.0f;
+  return __int_as_float(min(259 - e, 232) << 23);  // 2^(5 - (e - 127))
 }
 
 __device__ __forceinline__ float min3(float a, float b, float c) {
@@ -747,7 +768,8 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
   uint64_t *mmadone = accempty + W;      // every issued MMA has completed
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mmadone + 1);
   float *s_cmax = reinterpret_cast<float *>(tmem_slot + 1);    // [kGroupWarps]
-  unsigned *s_count = reinterpret_cast<unsigned *>(s_cmax + kGroupWarps);
+  float *s_top = s_cmax + kGroupWarps;                         // [kGroupWarps]
+  unsigned *s_count = reinterpret_cast<unsigned *>(s_top + kGroupWarps);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles = (static_cast<int64_t>(a.np) + kTP - 1) / kTP;
@@ -798,10 +820,30 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
     for (const CUtensorMap &m : tm.m) prefetch_tmap(&m);
     for (int c = 0; c < min(SA, group_tiles(warp) * nb); ++c) load(warp);
   }
+  float scale = 1.0f;  // (the point groups')
   if (warp >= 4) {
-    // the centroids' planes (of -2c; K-major, 64-byte swizzle), norms
-    // (+inf past k: never taken) and this warp's largest norm; eight lanes a
-    // centroid, two dimensions each at a time
+    // the centroids' largest magnitude (an infinite one leaves no finite
+    // margin, NaN is never taken)
+    float top = 0.0f;
+    const int t = static_cast<int>(threadIdx.x) - 128, kd = a.k * a.d;
+    const int quads = (reinterpret_cast<uintptr_t>(a.cent) & 15u) == 0 ? kd / 4 : 0;
+#pragma unroll 8
+    for (int e = t; e < quads; e += 32 * kGroupWarps) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(a.cent) + e);
+      top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+#pragma unroll 8
+    for (int e = 4 * quads + t; e < kd; e += 32 * kGroupWarps) top = fmaxf(top, fabsf(a.cent[e]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane == 0) s_top[warp - 4] = top;
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kGroupWarps) : "memory");
+#pragma unroll
+    for (int i = 0; i < kGroupWarps; ++i) top = fmaxf(top, s_top[i]);
+    scale = km_scale(top);
+    // the planes of -2c s (K-major, 64-byte swizzle), norms of c s (+inf past
+    // k: never taken) and this warp's largest norm; eight lanes a centroid,
+    // two dimensions each at a time
     const int sub = lane & 7;
     float cmax = 0.0f;
     for (int c = 4 * (warp - 4) + (lane >> 3); c < kp; c += 4 * kGroupWarps) {
@@ -809,13 +851,13 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       float sq = 0.0f;
 #pragma unroll 4
       for (int j = 2 * sub; j < 32 * nb; j += 16) {
-        const float v0 = c < a.k && j < a.d ? row[j] : 0.0f;
-        const float v1 = c < a.k && j + 1 < a.d ? row[j + 1] : 0.0f;
+        const float v0 = c < a.k && j < a.d ? row[j] * scale : 0.0f;
+        const float v1 = c < a.k && j + 1 < a.d ? row[j + 1] * scale : 0.0f;
         sq = fmaf(v0, v0, sq);
         sq = fmaf(v1, v1, sq);
-        const uint32_t hi = km_bf16x2(-2.0f * v0, -2.0f * v1);
-        const float2 h = km_bf16_pair(hi);
-        const uint32_t lo = km_bf16x2(__fsub_rn(-2.0f * v0, h.x), __fsub_rn(-2.0f * v1, h.y));
+        const uint32_t hi = km_f16x2(-2.0f * v0, -2.0f * v1);
+        const float2 h = km_f16_pair(hi);
+        const uint32_t lo = km_f16x2(__fsub_rn(-2.0f * v0, h.x), __fsub_rn(-2.0f * v1, h.y));
         const int w = (j & 31) >> 1;  // 32-bit word of the 64-byte row
         const int off = (j >> 5) * bblock + c * 64 + (((w >> 2) ^ ((c >> 1) & 3)) << 4) +
                         ((w & 3) << 2);
@@ -845,7 +887,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       const int g = warp;
       const uint32_t tacc = tmem + static_cast<uint32_t>(g * (512 / W));
       const uint32_t tA = tacc + static_cast<uint32_t>(NC);
-      const uint32_t idesc = idesc_bf16(NC);
+      const uint32_t idesc = idesc_f16(NC);
       const int ksteps = (a.d + 15) / 16;
       const int nt = group_tiles(g);
       int item = 0;          // passes issued
@@ -914,7 +956,14 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
 #pragma unroll
     for (int i = 0; i < kGroupWarps; ++i) cmax = fmaxf(cmax, s_cmax[i]);
     const double nu = (a.d + 4) * 0x1p-24;
-    const float bound = static_cast<float>((16.0 * nu / (1.0 - nu) + 0x1p-15) * 1.001);
+    const float bound = static_cast<float>((16.0 * nu / (1.0 - nu) + 0x1p-19) * 1.001);
+    // (in scaled units) sums of norms from which everything is a candidate --
+    // near the end of FP32's range unscaled, or of FP16's -- and what the
+    // margin is at least
+    const float most = fminf(1e36f * scale * scale, 0x1p31f);
+    const float least = 1e-37f * scale * scale;
+    const float inv = 1.0f / scale;  // a power of two too
+    const float2 scale2 = make_float2(scale, scale);
     [[maybe_unused]] const int e_w = AU ? a.e[w4] : 0;
 
     // Splits the next block of the group's sequence into its TMEM stage and
@@ -960,10 +1009,11 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       uint32_t hi[16], lo[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
+        x[i] = __fmul2_rn(x[i], scale2);
         xn = __ffma2_rn(x[i], x[i], xn);
-        hi[i] = km_bf16x2(x[i].x, x[i].y);
-        const float2 r = __ffma2_rn(km_bf16_pair(hi[i]), make_float2(-1.0f, -1.0f), x[i]);
-        lo[i] = km_bf16x2(r.x, r.y);
+        hi[i] = km_f16x2(x[i].x, x[i].y);
+        const float2 r = __ffma2_rn(km_f16_pair(hi[i]), make_float2(-1.0f, -1.0f), x[i]);
+        lo[i] = km_f16x2(r.x, r.y);
       }
       const uint32_t dst = tA + static_cast<uint32_t>(s * kTcStageCols);
       tmem_st16(dst, hi);
@@ -993,8 +1043,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       if (!ok) break;
       const float xsum = xn.x + xn.y + cmax;
       xn = xnext;
-      // sums near the end of FP32's range: everything is a candidate
-      const float margin = xsum < 1e36f ? bound * xsum + 1e-37f : INFINITY;
+      const float margin = xsum < most ? bound * xsum + least : INFINITY;
       float g1 = INFINITY;  // the smallest g of the passes so far
       int k1 = 0;           // its centroid, when the only candidate
       bool close = true;
@@ -1056,7 +1105,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       if (!ok) break;
       const int64_t p = (blockIdx.x + (g + static_cast<int64_t>(it) * W) * gridDim.x) * kTP + m;
       const bool live = p < a.np;
-      const float lim = margin < INFINITY ? g1 + margin : INFINITY;
+      const float lim = margin < INFINITY ? (g1 + margin) * inv * inv : INFINITY;
       close = live && (close || !(lim < INFINITY));
       if (live && !close) a.out[p] = static_cast<uint32_t>(k1);
       const unsigned vote = __ballot_sync(0xffffffffu, close);
@@ -1087,6 +1136,9 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
   float *cs = reinterpret_cast<float *>(smem);
   for (int c = warp; c < a.k; c += km_tc_threads(W) / 32)
     for (int j = lane; j < a.d; j += 32) cs[c * (a.d + 1) + j] = a.cent[static_cast<int64_t>(c) * a.d + j];
+  if (warp >= 4)
+    for (int c = static_cast<int>(threadIdx.x) - 128; c < a.k; c += 32 * kGroupWarps)
+      cn[c] = cn[c] / scale / scale;  // the norms unscaled
   __syncthreads();
   if (warp < 4) return;
   float *xs = cs + a.k * (a.d + 1) + (warp - 4) * a.d;
@@ -1301,7 +1353,7 @@ bool km_tc_plan(const float *points, int np, int d, int k, KmTcPlan *out) {
   if (p.sa < 2) return false;
   const int bars = p.W * (p.sa + 2 * p.stages + 2) + 1;
   p.smem = 1024 + p.W * p.sa * slot + planes(p.kp) + static_cast<size_t>(p.kp) * 4 + bars * 8 +
-           (1 + 4 * p.W + 1) * 4 + 16;
+           (1 + 8 * p.W + 1) * 4 + 16;
   // the close calls' centroids and point rows reuse the ring and the planes
   const size_t settle = (static_cast<size_t>(k) * (d + 1) + 4 * p.W * static_cast<size_t>(d)) * 4;
   if (settle > p.W * p.sa * slot + planes(p.kp) || p.smem > 227 * 1024) return false;
