@@ -155,6 +155,9 @@ __device__ __forceinline__ void push_close(unsigned *ccount, uint2 *citems, int6
 // the reference's distance of its candidates and keeps the first smallest
 // below FLT_MAX; the warp then keeps the smallest distance, the lowest index
 // among equal ones -- the first minimum in k order, the reference's pick.
+// xs lies on a 16-byte boundary: the warp reads it four elements a load.  The
+// loads bound the settling: 1M x 32 points, k = 64, all of them close calls
+// 1363 us, 1558 one element a load.
 __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, const float *cs,
                                                     int k, const float *cn, float lim) {
   const int lane = threadIdx.x & 31, st = d + 1;
@@ -163,15 +166,32 @@ __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, cons
   for (int c = lane; c < k; c += 32) {
     const float *cp = cs + c * st;
     if (lim < INFINITY) {
-      float dot[4] = {};
+      float dot = 0.0f;
       int j = 0;
-      for (; j + 4 <= d; j += 4)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) dot[u] = fmaf(xs[j + u], cp[j + u], dot[u]);
-      for (; j < d; ++j) dot[0] = fmaf(xs[j], cp[j], dot[0]);
-      if (!(fmaf(-2.0f, (dot[0] + dot[1]) + (dot[2] + dot[3]), cn[c]) <= lim)) continue;
+      for (; j + 4 <= d; j += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(xs + j);
+        dot = fmaf(v.x, cp[j], dot);
+        dot = fmaf(v.y, cp[j + 1], dot);
+        dot = fmaf(v.z, cp[j + 2], dot);
+        dot = fmaf(v.w, cp[j + 3], dot);
+      }
+      for (; j < d; ++j) dot = fmaf(xs[j], cp[j], dot);
+      if (!(fmaf(-2.0f, dot, cn[c]) <= lim)) continue;
     }  // else: every centroid is a candidate (see exact_pick)
-    const float dist = ref_dist(xs, cp, d);
+    float dist = 0.0f;  // ref_dist
+    auto add = [&](float x, float y) {
+      const float delta = __fsub_rn(x, y);
+      dist = __fmaf_rn(delta, delta, dist);
+    };
+    int j = 0;
+    for (; j + 4 <= d; j += 4) {
+      const float4 v = *reinterpret_cast<const float4 *>(xs + j);
+      add(v.x, cp[j]);
+      add(v.y, cp[j + 1]);
+      add(v.z, cp[j + 2]);
+      add(v.w, cp[j + 3]);
+    }
+    for (; j < d; ++j) add(xs[j], cp[j]);
     if (dist < bd) {
       bd = dist;
       bk = c;
@@ -191,23 +211,24 @@ __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, cons
 
 // Shared-memory floats the settle kernel stages (0: the centroids do not fit
 // in 96 KB and are read from global memory): centroids with rows of d + 1,
-// their norms, one point row per warp (8 warps).
+// their norms, one point row per warp (8 warps), each on a 16-byte boundary.
+__host__ __device__ constexpr int64_t up4(int64_t n) { return (n + 3) / 4 * 4; }
 __host__ __device__ constexpr int64_t settle_smem_floats(int k, int d) {
-  return static_cast<int64_t>(k) * (d + 1) + k + 8 * static_cast<int64_t>(d);
+  return up4(static_cast<int64_t>(k) * (d + 1) + k) + 8 * up4(d);
 }
-constexpr int64_t kSettleSmemFloats = 96 * 1024 / 4;
+constexpr int64_t kSettleSmemFloats = 96 * 1024 / 4 + 27;  // (27: all that the rounding adds)
 
 __global__ void __launch_bounds__(256) kmeans_settle_kernel(
     const float *points, int d, const float *cent, int k, const float *cnorm,
     const unsigned *ccount, const uint2 *citems, uint32_t *out, unsigned *exact, int staged) {
-  extern __shared__ float s_set[];
+  extern __shared__ __align__(16) float s_set[];
   const unsigned n = *ccount;
   if (exact && n && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(exact, n);
   const unsigned wpb = blockDim.x >> 5, warps = gridDim.x * wpb;
   if (blockIdx.x * wpb >= n) return;  // no entry for this block's warps
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float *cs = s_set, *cn = s_set + static_cast<int64_t>(k) * (d + 1);
-  float *xs = cn + k + wib * d;
+  float *xs = s_set + up4(static_cast<int64_t>(k) * (d + 1) + k) + wib * up4(d);
   if (staged) {
     for (int e = threadIdx.x; e < k * d; e += blockDim.x) {
       const int c = e / d, j = e - c * d;
@@ -1141,7 +1162,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
       cn[c] = cn[c] / scale / scale;  // the norms unscaled
   __syncthreads();
   if (warp < 4) return;
-  float *xs = cs + a.k * (a.d + 1) + (warp - 4) * a.d;
+  float *xs = cs + up4(a.k * (a.d + 1)) + (warp - 4) * up4(a.d);
   for (unsigned i = warp - 4; i < n; i += kGroupWarps) {
     const uint2 it = a.citems[static_cast<int64_t>(blockIdx.x) * a.list + i];
     const float *x = a.points + static_cast<int64_t>(it.x) * a.d;
@@ -1355,7 +1376,7 @@ bool km_tc_plan(const float *points, int np, int d, int k, KmTcPlan *out) {
   p.smem = 1024 + p.W * p.sa * slot + planes(p.kp) + static_cast<size_t>(p.kp) * 4 + bars * 8 +
            (1 + 8 * p.W + 1) * 4 + 16;
   // the close calls' centroids and point rows reuse the ring and the planes
-  const size_t settle = (static_cast<size_t>(k) * (d + 1) + 4 * p.W * static_cast<size_t>(d)) * 4;
+  const size_t settle = static_cast<size_t>(up4(static_cast<int64_t>(k) * (d + 1)) + 4 * p.W * up4(d)) * 4;
   if (settle > p.W * p.sa * slot + planes(p.kp) || p.smem > 227 * 1024) return false;
   p.smem = std::max<size_t>(p.smem, 120 * 1024);  // one CTA per SM: all 512 TMEM columns
   *out = p;
