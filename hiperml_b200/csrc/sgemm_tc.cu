@@ -95,6 +95,13 @@ enum AMode : int {
 };
 __host__ __device__ constexpr bool am_kcontig(int am) { return am == kAK || am == kAKU; }
 __host__ __device__ constexpr bool am_unaligned(int am) { return am >= kAMU; }
+// The unaligned forms, which take the place of FP32 tiles, scale both operands
+// by 2^16 before they are split: the third BF16 plane of an element below 2^-110
+// would otherwise need bits below BF16's smallest subnormal, 2^-133 (with the
+// scale every FP32 value, 2^-149 itself included, splits exactly).  Sums carry
+// 2^32 until they are stored; one that leaves FP32's range for it is formed
+// again in plain FP32 like every sum that is not finite.
+constexpr float kAUScale = 0x1p16f, kAUUnscale = 0x1p-32f;
 // The maps of A (one, or one per class) and the class offsets e_r.
 template <int AM>
 struct AMaps {
@@ -334,7 +341,7 @@ struct SplitWalk {
 // lo = TF32(x - hi).
 template <int NS>
 __global__ void split_b_kernel(const float *B, int64_t sbk, int64_t sbn, int K, int N,
-                               void *planes_out, int k_pad, int n_pad) {
+                               void *planes_out, int k_pad, int n_pad, float scale) {
   // the tensor-core kernel that reads the planes is launched as a
   // programmatic dependent: its set-up and A loads overlap this kernel
   allow_dependent_launch();
@@ -348,7 +355,7 @@ __global__ void split_b_kernel(const float *B, int64_t sbk, int64_t sbn, int K, 
     for (int j = 0; j < 8; ++j) {
       const int k = k0 + j;
       x[j] = (n < N && k < K)
-                 ? B[static_cast<int64_t>(k) * sbk + static_cast<int64_t>(n) * sbn]
+                 ? scale * B[static_cast<int64_t>(k) * sbk + static_cast<int64_t>(n) * sbn]
                  : 0.0f;
     }
     if constexpr (NS == 4) {
@@ -842,6 +849,14 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
 #pragma unroll
         for (int k = 0; k < 32; ++k) x[k] = a32[k * kBM + m];
       }
+      if constexpr (AU) {
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+          const float2 t = __fmul2_rn(make_float2(x[k], x[k + 1]), make_float2(kAUScale, kAUScale));
+          x[k] = t.x;
+          x[k + 1] = t.y;
+        }
+      }
       uint32_t wv[16];
       [[maybe_unused]] uint32_t wl[16];
       [[maybe_unused]] int sexp_m = 0;
@@ -1049,7 +1064,10 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
           // the warp's scratch row
           bool odd = false;
 #pragma unroll
-          for (int c = 0; c < DC; ++c) odd |= !(fabsf(sums[c]) <= FLT_MAX);
+          for (int c = 0; c < DC; ++c) {
+            odd |= !(fabsf(sums[c]) <= FLT_MAX);
+            sums[c] *= kAUUnscale;  // (infinities and NaN stay)
+          }
           float *row = scratch + (warp - kDrainWarp0) * DC;
           for (unsigned todo = __ballot_sync(0xffffffffu, ok && odd && gm < p.M); todo;
                todo &= todo - 1) {
@@ -1100,6 +1118,10 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
         for (int i = 0; i < DC; ++i) sums[i] = 0.0f;
       }
       if (split > 1 || AU) {
+        if constexpr (AU) {
+#pragma unroll
+          for (int i = 0; i < DC; ++i) sums[i] *= kAUUnscale;
+        }
 #pragma unroll
         for (int i = 0; i < DC; ++i) red[(d * DC + i) * kBM + m] = sums[i];
         if constexpr (AU) {
@@ -1428,11 +1450,12 @@ bool tail_buffers(cudaStream_t s, TcWalk *w) {
 // B -> BF16 planes in `planes` ([NS][n_pad][k_pad]).
 template <int NS>
 hml_status split_b(const GemmProblem &p, __nv_bfloat16 *planes, int k_pad, int n_pad,
-                   cudaStream_t s) {
+                   cudaStream_t s, float scale = 1.0f) {
   const int64_t chunks = static_cast<int64_t>(n_pad) * (k_pad / 8);
   const int blocks = static_cast<int>(std::min<int64_t>((chunks + 255) / 256, 4 * sm_count()));
   count_launch();
-  split_b_kernel<NS><<<blocks, 256, 0, s>>>(p.B, p.sbk, p.sbn, p.K, p.N, planes, k_pad, n_pad);
+  split_b_kernel<NS><<<blocks, 256, 0, s>>>(p.B, p.sbk, p.sbn, p.K, p.N, planes, k_pad, n_pad,
+                                          scale);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     note_cuda_error(e, "split_b");
@@ -1486,7 +1509,7 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
     return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s,
                                         bexp);
   } else {
-    st = split_b<NS>(p, planes, k_pad, n_pad, s);
+    st = split_b<NS>(p, planes, k_pad, n_pad, s, am_unaligned(AM) ? kAUScale : 1.0f);
     if (st != HML_STATUS_SUCCESS) return st;
     if constexpr (NS <= 3) {
       if (persist)
