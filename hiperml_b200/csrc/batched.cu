@@ -456,27 +456,26 @@ hml_status batch_plan_create(hml_order order, const hml_gemm_desc *descs, int co
 // most SMs idle: before the split-BF16 part it added 68 us to the 258 of 60
 // uneven problems, beside it 13.
 hml_status launch_plan(BatchPlan *pl, cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
   const bool beside = pl->side != nullptr;
-  if (pl->nitems > 0) {
-    cudaStream_t t = s;
-    if (beside) {
-      t = pl->side;
-      e = cudaEventRecord(pl->fork, s);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(t, pl->fork, 0);
-    }
-    if (e == cudaSuccess) {
-      count_launch();
-      e = launch_batched(pl->args, pl->ctas, t);
-    }
-    if (beside && e == cudaSuccess) e = cudaEventRecord(pl->join, t);
-    note_cuda_error(e, "batched launch");
+  cudaStream_t t = s;
+  cudaError_t e = cudaSuccess;
+  if (beside) {
+    t = pl->side;
+    e = cudaEventRecord(pl->fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(t, pl->fork, 0);
+    note_cuda_error(e, "batched fork");
     if (e != cudaSuccess) return HML_STATUS_CUDA_ERROR;
   }
-  const hml_status st = tc_batch_launch(pl->tc, s);
+  if (pl->nitems > 0) {
+    count_launch();
+    e = launch_batched(pl->args, pl->ctas, t);
+    note_cuda_error(e, "batched launch");
+  }
+  const hml_status st = e == cudaSuccess ? tc_batch_launch(pl->tc, s) : HML_STATUS_CUDA_ERROR;
   if (beside) {
     // joined whatever the launches returned: a capture must not end forked
-    e = cudaStreamWaitEvent(s, pl->join, 0);
+    e = cudaEventRecord(pl->join, t);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, pl->join, 0);
     note_cuda_error(e, "batched join");
   }
   return st != HML_STATUS_SUCCESS ? st : cuda_status(e);
