@@ -16,6 +16,7 @@ hml_status fill_random(float *out, size_t n, uint64_t seed, uint64_t stream_id, 
 hml_status sgemm_error_fp64(const GemmProblem &p, const float *C0, double err[4], cudaStream_t s);
 hml_status release_all();
 void release_host_staging();
+void release_spare_branches();
 int simt_num_shapes();
 void simt_shape(int v, int *bm, int *bn, int *wk);
 int tc_num_shapes();
@@ -406,6 +407,7 @@ hml_status hml_check_wait_limit(void *stream) {
 
 hml_status hml_release_resources(void) {
   release_host_staging();
+  release_spare_branches();
   return release_all();
 }
 

@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <vector>
@@ -248,6 +249,74 @@ double tile_cost(int bn, int K) {
 
 }  // namespace
 
+namespace {
+
+// A stream and two events with which a plan runs one part beside the other.
+struct Branch {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+
+void branch_destroy(Branch *b) {
+  if (b->fork) cudaEventDestroy(b->fork);
+  if (b->join) cudaEventDestroy(b->join);
+  if (b->stream) cudaStreamDestroy(b->stream);
+  *b = Branch();
+}
+
+// Branches of destroyed plans, kept for the next ones: creating a stream takes
+// about 400 us where the driver has to set up a queue for it (a whole plan of 60
+// problems 600).  Each belongs to one plan at a time; at most kSpareBranches are
+// kept, until hml_release_resources.
+constexpr int kSpareBranches = 16;
+std::mutex g_branch_mu;
+struct {
+  int device;
+  Branch b;  // no stream: a free place
+} g_spare[kSpareBranches];
+
+hml_status branch_take(int device, Branch *out) {
+  {
+    std::lock_guard<std::mutex> lk(g_branch_mu);
+    for (auto &sp : g_spare) {
+      if (!sp.b.stream || sp.device != device) continue;
+      *out = sp.b;
+      sp.b = Branch();
+      // (a plan destroyed inside a capture leaves its stream in it)
+      if (!stream_capturing(out->stream)) return HML_STATUS_SUCCESS;
+      branch_destroy(out);
+    }
+  }
+  Branch b;
+  cudaError_t e = cudaStreamCreateWithFlags(&b.stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    note_cuda_error(e, "batch plan stream");
+    branch_destroy(&b);
+    return HML_STATUS_CUDA_ERROR;
+  }
+  *out = b;
+  return HML_STATUS_SUCCESS;
+}
+
+void branch_give(int device, Branch *b) {
+  if (!b->stream) return;
+  {
+    std::lock_guard<std::mutex> lk(g_branch_mu);
+    for (auto &sp : g_spare) {
+      if (sp.b.stream) continue;
+      sp.device = device;
+      sp.b = *b;
+      *b = Branch();
+      return;
+    }
+  }
+  branch_destroy(b);
+}
+
+}  // namespace
+
 // Host-side plan (opaque to callers).
 struct BatchPlan {
   int device = -1;
@@ -258,9 +327,7 @@ struct BatchPlan {
   void *dev = nullptr;  // [queue 256 B][problems][items]
   BatchArgs args = {};
   TcBatch *tc = nullptr;  // the split-BF16 part
-  // the SIMT part's branch, where the plan has both parts
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  Branch side;            // the SIMT part's, once both parts have run side by side
   cudaStream_t capture_stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -436,48 +503,80 @@ hml_status batch_plan_create(hml_order order, const hml_gemm_desc *descs, int co
   pl->args.probs = reinterpret_cast<const BatchProblem *>(base + op);
   pl->args.items = reinterpret_cast<const BatchItem *>(base + oi);
   pl->args.nitems = pl->nitems;
-  if (pl->nitems > 0 && tc_batch_items(pl->tc) > 0) {
-    e = cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&pl->fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&pl->join, cudaEventDisableTiming);
-    if (e != cudaSuccess) {
-      note_cuda_error(e, "batch plan stream");
-      batch_plan_destroy(pl);
-      return HML_STATUS_CUDA_ERROR;
-    }
-  }
   *out = pl;
   return HML_STATUS_SUCCESS;
 }
 
-// The plan's launches: the SIMT queue beside the split-BF16 part, on the
-// plan's own stream between two events (branches of the graph when captured).
-// The SIMT part is a few problems of at most 8 columns whose long tiles leave
-// most SMs idle: before the split-BF16 part it added 68 us to the 258 of 60
-// uneven problems, beside it 13.
+namespace {
+
+hml_status launch_simt_part(const BatchPlan *pl, cudaStream_t s) {
+  count_launch();
+  const cudaError_t e = launch_batched(pl->args, pl->ctas, s);
+  note_cuda_error(e, "batched launch");
+  return cuda_status(e);
+}
+
+hml_status launch_parts_in_turn(const BatchPlan *pl, cudaStream_t s) {
+  hml_status st = HML_STATUS_SUCCESS;
+  if (pl->nitems > 0) st = launch_simt_part(pl, s);
+  return st == HML_STATUS_SUCCESS ? tc_batch_launch(pl->tc, s) : st;
+}
+
+// Both parts captured as branches: the split-BF16 part depends on what the SIMT
+// part depended on, what follows on both.  Set on the capture itself, without a
+// second stream.
+hml_status capture_parts(const BatchPlan *pl, cudaStream_t s) {
+  std::vector<cudaGraphNode_t> before, simt;
+  auto read = [s](std::vector<cudaGraphNode_t> *nodes) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v2(s, &cs, nullptr, nullptr, &deps, &n) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusActive) {
+      cudaGetLastError();
+      return false;
+    }
+    nodes->assign(deps, deps + n);
+    return true;
+  };
+  if (!read(&before)) return launch_parts_in_turn(pl, s);
+  hml_status st = launch_simt_part(pl, s);
+  if (st != HML_STATUS_SUCCESS || !read(&simt)) return HML_STATUS_CUDA_ERROR;
+  cudaError_t e = cudaStreamUpdateCaptureDependencies(s, before.data(), before.size(),
+                                                      cudaStreamSetCaptureDependencies);
+  if (e == cudaSuccess) {
+    st = tc_batch_launch(pl->tc, s);
+    e = cudaStreamUpdateCaptureDependencies(s, simt.data(), simt.size(),
+                                            cudaStreamAddCaptureDependencies);
+  }
+  note_cuda_error(e, "batched capture");
+  return st != HML_STATUS_SUCCESS ? st : cuda_status(e);
+}
+
+}  // namespace
+
+// The plan's launches: the SIMT queue beside the split-BF16 part -- branches of
+// the graph when captured, else on a stream of the plan's own, taken by the
+// first such run, between two events.  The SIMT part is a few problems of at
+// most 8 columns whose long tiles leave most SMs idle: before the split-BF16
+// part it added 68 us to the 258 of 60 uneven problems, beside it 13.
 hml_status launch_plan(BatchPlan *pl, cudaStream_t s) {
-  const bool beside = pl->side != nullptr;
-  cudaStream_t t = s;
-  cudaError_t e = cudaSuccess;
-  if (beside) {
-    t = pl->side;
-    e = cudaEventRecord(pl->fork, s);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(t, pl->fork, 0);
-    note_cuda_error(e, "batched fork");
-    if (e != cudaSuccess) return HML_STATUS_CUDA_ERROR;
-  }
-  if (pl->nitems > 0) {
-    count_launch();
-    e = launch_batched(pl->args, pl->ctas, t);
-    note_cuda_error(e, "batched launch");
-  }
-  const hml_status st = e == cudaSuccess ? tc_batch_launch(pl->tc, s) : HML_STATUS_CUDA_ERROR;
-  if (beside) {
-    // joined whatever the launches returned: a capture must not end forked
-    e = cudaEventRecord(pl->join, t);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, pl->join, 0);
-    note_cuda_error(e, "batched join");
-  }
+  if (pl->nitems == 0 || tc_batch_items(pl->tc) == 0) return launch_parts_in_turn(pl, s);
+  if (stream_capturing(s)) return capture_parts(pl, s);
+  if (!pl->side.stream && branch_take(pl->device, &pl->side) != HML_STATUS_SUCCESS)
+    return launch_parts_in_turn(pl, s);
+  const Branch &b = pl->side;
+  cudaError_t e = cudaEventRecord(b.fork, s);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(b.stream, b.fork, 0);
+  note_cuda_error(e, "batched fork");
+  if (e != cudaSuccess) return HML_STATUS_CUDA_ERROR;
+  // from here on joined whatever a launch returns: s waits for what was put
+  // beside it
+  hml_status st = launch_simt_part(pl, b.stream);
+  if (st == HML_STATUS_SUCCESS) st = tc_batch_launch(pl->tc, s);
+  e = cudaEventRecord(b.join, b.stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b.join, 0);
+  note_cuda_error(e, "batched join");
   return st != HML_STATUS_SUCCESS ? st : cuda_status(e);
 }
 
@@ -523,12 +622,15 @@ void batch_plan_destroy(BatchPlan *pl) {
   if (pl->exec) cudaGraphExecDestroy(pl->exec);
   if (pl->graph) cudaGraphDestroy(pl->graph);
   if (pl->capture_stream) cudaStreamDestroy(pl->capture_stream);
-  if (pl->fork) cudaEventDestroy(pl->fork);
-  if (pl->join) cudaEventDestroy(pl->join);
-  if (pl->side) cudaStreamDestroy(pl->side);
+  branch_give(pl->device, &pl->side);
   if (pl->dev) cudaFree(pl->dev);
   tc_batch_destroy(pl->tc);
   delete pl;
+}
+
+void release_spare_branches() {
+  std::lock_guard<std::mutex> lk(g_branch_mu);
+  for (auto &sp : g_spare) branch_destroy(&sp.b);
 }
 
 // One-shot batch: the plan lives in stream-ordered memory for one launch.
