@@ -173,10 +173,11 @@ __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
 // lanes' loads to return nor keeps their use from being scheduled behind it,
 // and TMA refills the slot at once (a build with registers to spare did so,
 // and lost rows).  A slot is released after the block's first TMEM store,
-// which takes words of values from all of the row -- except in a ring of 2
+// which takes words of values from all of the row -- except in a ring of 2 or 4
 // slots (EARLY), which cannot wait for the operand stage that store needs
-// (8192^3 5.95 ms, 6.58 with the later release): there the arriving lane
-// comes from a vote on words w computed from every value.
+// (8192^3 with 2 slots 5.95 ms, 6.58 with the later release; 18944 x 64 x 4096
+// with 4 74.8 us, 77.0): there the arriving lane comes from a vote on words w
+// computed from every value.
 template <int N>
 __device__ __forceinline__ void release_early(uint64_t *bar, const uint32_t (&w)[N], int lane) {
   uint32_t all = w[0];
@@ -1269,7 +1270,7 @@ struct TcWalk {
 template <int BN, int NS, int AM, bool PERSIST = false>
 hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
                             const __nv_bfloat16 *planes, int k_pad, int n_pad, int *err,
-                            cudaStream_t s, const int *bexp = nullptr,
+                            cudaStream_t s, bool automatic, const int *bexp = nullptr,
                             const TcWalk *walk = nullptr) {
   if (NS == 5 && !bexp) return HML_STATUS_INVALID_VALUE;
   AMaps<AM> ta;
@@ -1309,17 +1310,18 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   const int kchunks = k_pad / kChunkK;
   args.kc = ((kchunks + c.split_k - 1) / c.split_k) * kChunkK;
   TcPlan plan;
-  // slots are held until the operand stage is free (release_early): rings of 4
-  // get 6 where that fits (18944 x 64 x 4096, 4 slots: 74.8 us when released
-  // earlier, 77.0, 74.3 with 6), and the persistent form, which only the
-  // automatic choice reaches, has no use for one of 2
-  int sa = c.stages;
-  if (sa == 4 || (PERSIST && sa == 2)) {
-    const int given = sa;
-    for (sa = 6; sa > given && !tc_plan(BN, NS, sa, &plan, AM); sa -= 2) {
-    }
+  // A ring runs as deep as the configuration says; on the automatic path one of
+  // 4 gets 6 where that fits and costs no operand stage (BF16X6, K = 4096, a
+  // wave of row tiles, us with 4 and 6 slots: N = 16 74.7, 70.7; 64 76.9, 71.7;
+  // 128 96, 97), and the persistent form, which only that path reaches and
+  // whose slots are held until the operand stage is free (release_early), has
+  // no use for one of 2.
+  if (!tc_plan(BN, NS, c.stages, &plan, AM)) return HML_STATUS_INVALID_VALUE;
+  if (automatic && (plan.sa == 4 || (PERSIST && plan.sa == 2))) {
+    TcPlan deeper;
+    for (int sa = 6; sa > plan.sa; sa -= 2)
+      if (tc_plan(BN, NS, sa, &deeper, AM) && deeper.so >= plan.so) plan = deeper;
   }
-  if (!tc_plan(BN, NS, sa, &plan, AM)) return HML_STATUS_INVALID_VALUE;
   args.sa = plan.sa;
   args.so = plan.so;
   args.n_pad = n_pad;
@@ -1327,7 +1329,7 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   args.bexp = bexp;
   const size_t smem = tc_plan_bytes(BN, NS, plan, AM);
   void (*kern)(AMaps<AM>, CUtensorMap, TcArgs) =
-      plan.sa == 2 ? tc_kernel<BN, NS, AM, PERSIST, !PERSIST && !am_unaligned(AM)>
+      plan.sa <= 4 ? tc_kernel<BN, NS, AM, PERSIST, !PERSIST && !am_unaligned(AM)>
                    : tc_kernel<BN, NS, AM, PERSIST, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
@@ -1382,7 +1384,8 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
   const int64_t slots = sm_count();
   const int64_t full = (tiles / slots) * slots;
   const int split = c.split_k == 1 && n_pad == BN ? tail_split(tiles, slots, k_pad) : 1;
-  if (split == 1) return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, err, s);
+  if (split == 1)
+    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, err, s, true);
   const int64_t m1 = full * kBM;
   GemmProblem head = p, tail = p;
   head.M = static_cast<int>(m1);
@@ -1391,9 +1394,9 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
   tail.C = p.C + m1 * p.scm;
   hml_sgemm_config ct = c;
   ct.split_k = split;
-  hml_status st = launch_tc_planes<BN, NS, AM>(head, c, planes, k_pad, n_pad, err, s);
+  hml_status st = launch_tc_planes<BN, NS, AM>(head, c, planes, k_pad, n_pad, err, s, true);
   if (st != HML_STATUS_SUCCESS) return st;
-  return launch_tc_planes<BN, NS, AM>(tail, ct, planes, k_pad, n_pad, err, s);
+  return launch_tc_planes<BN, NS, AM>(tail, ct, planes, k_pad, n_pad, err, s, true);
 }
 
 // The persistent form's work for a split_k = 1 configuration on the automatic
@@ -1507,18 +1510,19 @@ hml_status run_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t 
     st = split_b_fh(p, ws, bexp, k_pad, n_pad, s);
     if (st != HML_STATUS_SUCCESS) return st;
     return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s,
-                                        bexp);
+                                        waves, bexp);
   } else {
     st = split_b<NS>(p, planes, k_pad, n_pad, s, am_unaligned(AM) ? kAUScale : 1.0f);
     if (st != HML_STATUS_SUCCESS) return st;
     if constexpr (NS <= 3) {
       if (persist)
         return launch_tc_planes<BN, NS, AM, true>(p, c, planes, k_pad, n_pad,
-                                                  device_error_word(), s, nullptr, &walk);
+                                                  device_error_word(), s, true, nullptr, &walk);
     }
     if (waves)
       return launch_tc_waves<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s);
-    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s);
+    return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, device_error_word(), s,
+                                        false);
   }
 }
 
@@ -2469,7 +2473,7 @@ hml_status run_tc_static(const GemmProblem &p, const hml_sgemm_config &c, const 
   auto *planes = static_cast<__nv_bfloat16 *>(a.scratch);
   hml_status st = split_b<NS>(p, planes, k_pad, n_pad, s);
   if (st != HML_STATUS_SUCCESS) return st;
-  return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, a.err, s);
+  return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, a.err, s, false);
 }
 
 template <int NS>
