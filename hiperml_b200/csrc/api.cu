@@ -236,14 +236,16 @@ hml_status hml_sgemm_ex(hml_order order, hml_op transA, hml_op transB, int M, in
   GemvProblem g;
   if (as_gemv(p, &g)) return launch_gemv(g, kGemvTuned, s);
   hml_sgemm_config c;
-  if (unaligned_config(p, &c, s)) {
+  bool unaligned;
+  st = select_auto(p, &c, &unaligned, s);
+  if (st == HML_STATUS_SUCCESS && unaligned) {
     st = launch_tc_unaligned(p, c, s);
     // no room for the planes of B, or none yet in a stream under capture: the
     // SIMT tiles, which need none
     if (st != HML_STATUS_ALLOC_FAILED) return st;
     cudaGetLastError();
+    st = select_config(p, &c, s);
   }
-  st = select_config(p, &c, s);
   if (st != HML_STATUS_SUCCESS) return st;
   return run_config(p, c, s, true);
 }

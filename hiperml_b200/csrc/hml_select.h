@@ -7,9 +7,9 @@
 
 namespace hml {
 hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s = nullptr);
-// The configuration hml_sgemm_ex runs a problem with an unaligned A with on the
-// tensor cores (launch_tc_unaligned); false when it takes select_config's.
-bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s);
+// The configuration hml_sgemm_ex runs: select_config's, or for an A that TMA
+// cannot address as it stands one for launch_tc_unaligned (*unaligned).
+hml_status select_auto(const GemmProblem &p, hml_sgemm_config *c, bool *unaligned, cudaStream_t s);
 hml_sgemm_config heuristic_config(const GemmProblem &p, int algo);
 hml_sgemm_config simt_config(const GemmProblem &p, int var);
 // A loaded reference v1 SGEMM rule for the row-major K x N class, mapped onto

@@ -214,22 +214,29 @@ hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t
 // from there on the error is no larger than SIMT's (RMS 0.7 to 0.9 of it over
 // N = 2 to 100, K = 101 to 3001), at K = 65 its maximum is (1.7e-7 against
 // 1.2e-7).
-bool unaligned_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t s) {
+//
+// A record that the program measured or loaded for exactly this shape stands if
+// it can run A as it is.  Else one selection serves both ways: the choice for
+// the same problem with an addressable A, which where it is SIMT and can read A
+// is also the choice among the configurations that can.
+hml_status select_auto(const GemmProblem &p, hml_sgemm_config *c, bool *unaligned,
+                       cudaStream_t s) {
+  *unaligned = false;
   const int64_t ld = p.a_kcontig() ? p.sam : p.sak;
   const bool base_ok = (reinterpret_cast<uintptr_t>(p.A) & 15u) == 0;
-  if ((base_ok && ld % 4 == 0) || !tc_unaligned_ok(p)) return false;
-  // the choice for the same problem with an addressable A
+  if ((base_ok && ld % 4 == 0) || !tc_unaligned_ok(p)) return select_config(p, c, s);
+  if (tuned_by_user(p, c) && check_config_ok(p, *c)) return HML_STATUS_SUCCESS;
   GemmProblem q = p;
   q.A = reinterpret_cast<const float *>(reinterpret_cast<uintptr_t>(p.A) & ~uintptr_t(15));
   (p.a_kcontig() ? q.sam : q.sak) = (ld + 3) / 4 * 4;
-  if (select_config(q, c, s) != HML_STATUS_SUCCESS) return false;
-  if (c->algo == HML_ALGO_BF16X6) return true;
+  if (select_config(q, c, s) != HML_STATUS_SUCCESS) return select_config(p, c, s);
   const double mk = static_cast<double>(p.M) * p.K;
   if (c->algo == HML_ALGO_SIMT &&
       (p.K < 100 || (mk * std::max(p.N, 8) < 0x1p25 && (p.M < 40 * 128 || mk * p.N < 0x1p24))))
-    return false;
-  *c = heuristic_config(q, HML_ALGO_BF16X6);
-  return true;
+    return check_config_ok(p, *c) ? HML_STATUS_SUCCESS : select_config(p, c, s);
+  if (c->algo != HML_ALGO_BF16X6) *c = heuristic_config(q, HML_ALGO_BF16X6);
+  *unaligned = true;
+  return HML_STATUS_SUCCESS;
 }
 
 }  // namespace hml

@@ -57,6 +57,7 @@ struct Key {
 struct Rec {
   hml_sgemm_config cfg;
   float us;
+  bool shipped = false;  // of the table that comes with the library
 };
 
 // GEMV records: layout (0 = rows of A contiguous, 1 = columns), P, Q
@@ -120,6 +121,9 @@ void load_default_table() {
   }
   int n = 0;
   tune_load(path.c_str(), &n);  // a missing file leaves the table empty
+  if (env && *env) return;
+  std::lock_guard<std::mutex> lk(g_mu);
+  for (auto &kv : g_table) kv.second.shipped = true;
 }
 }  // namespace
 
@@ -150,6 +154,15 @@ bool tuned_lookup(const GemmProblem &p, hml_sgemm_config *c) {
   // only trust neighbours within a factor ~2 in every dimension
   if (!pick || best > 3.0) return false;
   *c = pick->cfg;
+  return true;
+}
+
+bool tuned_by_user(const GemmProblem &p, hml_sgemm_config *c) {
+  load_default_table();
+  std::lock_guard<std::mutex> lk(g_mu);
+  const auto it = g_table.find(key_of(p));
+  if (it == g_table.end() || it->second.shipped || !allowed(it->second.cfg.algo)) return false;
+  *c = it->second.cfg;
   return true;
 }
 
