@@ -28,7 +28,6 @@
 #include <mutex>
 #include <map>
 #include <string>
-#include <system_error>
 #include <thread>
 
 #include "../../include/hml_sgemm.h"
@@ -147,8 +146,8 @@ class Team {
         sem_init(&sem_[threads_], 0, 0);
         thread_[threads_] = std::thread(&Team::loop, this, threads_);
       }
-    } catch (const std::system_error &) {
-      // as many as there are
+    } catch (...) {
+      // no thread or no memory for one: as many as there are
     }
     pthread_sigmask(SIG_SETMASK, &old, nullptr);
     fn_ = fn;
