@@ -740,6 +740,19 @@ __device__ __forceinline__ float2 km_f16_pair(uint32_t w) {
   return __half22float2(*reinterpret_cast<const __half2 *>(&w));
 }
 
+// x less the pair's values.
+__device__ __forceinline__ float2 km_residual(uint32_t w, float2 x) {
+  float2 r;
+  asm("{\n\t.reg .b16 h0, h1, m;\n\t"
+      "mov.b32 {h0, h1}, %2;\n\t"
+      "mov.b16 m, 0xBC00;\n\t"
+      "fma.rn.f32.f16 %0, h0, m, %3;\n\t"
+      "fma.rn.f32.f16 %1, h1, m, %4;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "r"(w), "f"(x.x), "f"(x.y));
+  return r;
+}
+
 // The power of two that brings magnitudes up to `top` (not NaN) below 2^6: at
 // most 2^105, so that 1 / s is normal (g of centroids that small all lie within
 // the margin's 1e-37), and 1 when there is nothing to scale.
@@ -813,6 +826,23 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
     fence_mbar_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (warp >= 4) {
+    // the centroids' largest magnitude (an infinite one leaves no finite
+    // margin, NaN is never taken)
+    float top = 0.0f;
+    const int t = static_cast<int>(threadIdx.x) - 128, kd = a.k * a.d;
+    const int quads = (reinterpret_cast<uintptr_t>(a.cent) & 15u) == 0 ? kd / 4 : 0;
+#pragma unroll 8
+    for (int e = t; e < quads; e += 32 * kGroupWarps) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(a.cent) + e);
+      top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+#pragma unroll 8
+    for (int e = 4 * quads + t; e < kd; e += 32 * kGroupWarps) top = fmaxf(top, fabsf(a.cent[e]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane == 0) s_top[warp - 4] = top;
+  }
   __syncthreads();
 
   // Loads the next block of group g's sequence (its tiles one after another,
@@ -843,22 +873,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
   }
   float scale = 1.0f;  // (the point groups')
   if (warp >= 4) {
-    // the centroids' largest magnitude (an infinite one leaves no finite
-    // margin, NaN is never taken)
-    float top = 0.0f;
-    const int t = static_cast<int>(threadIdx.x) - 128, kd = a.k * a.d;
-    const int quads = (reinterpret_cast<uintptr_t>(a.cent) & 15u) == 0 ? kd / 4 : 0;
-#pragma unroll 8
-    for (int e = t; e < quads; e += 32 * kGroupWarps) {
-      const float4 v = __ldg(reinterpret_cast<const float4 *>(a.cent) + e);
-      top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    }
-#pragma unroll 8
-    for (int e = 4 * quads + t; e < kd; e += 32 * kGroupWarps) top = fmaxf(top, fabsf(a.cent[e]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if (lane == 0) s_top[warp - 4] = top;
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * kGroupWarps) : "memory");
+    float top = s_top[0];
 #pragma unroll
     for (int i = 0; i < kGroupWarps; ++i) top = fmaxf(top, s_top[i]);
     scale = km_scale(top);
@@ -1033,7 +1048,7 @@ __global__ void __launch_bounds__(km_tc_threads(W), 1)
         x[i] = __fmul2_rn(x[i], scale2);
         xn = __ffma2_rn(x[i], x[i], xn);
         hi[i] = km_f16x2(x[i].x, x[i].y);
-        const float2 r = __ffma2_rn(km_f16_pair(hi[i]), make_float2(-1.0f, -1.0f), x[i]);
+        const float2 r = km_residual(hi[i], x[i]);
         lo[i] = km_f16x2(r.x, r.y);
       }
       const uint32_t dst = tA + static_cast<uint32_t>(s * kTcStageCols);
