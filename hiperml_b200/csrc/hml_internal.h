@@ -125,7 +125,6 @@ hml_status workspace_slot(int slot, size_t bytes, cudaStream_t s, void **ptr);
 // Whether a request would be met without an allocation, which a stream under
 // capture may not be able to make.
 bool workspace_held(int slot, size_t bytes, cudaStream_t s);
-bool tile_counters_held(size_t n, cudaStream_t s);
 bool stream_capturing(cudaStream_t s);
 // n zero-initialised counters private to (device, stream).  Kernels that use
 // them leave every counter at zero again when they finish.

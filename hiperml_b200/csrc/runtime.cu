@@ -120,13 +120,6 @@ bool workspace_held(int slot, size_t bytes, cudaStream_t s) {
   return it != g_ws[slot].end() && it->second.bytes >= bytes;
 }
 
-bool tile_counters_held(size_t n, cudaStream_t s) {
-  const int d = current_device();
-  std::lock_guard<std::mutex> lk(g_mu);
-  auto it = g_counters.find(std::make_pair(d, s));
-  return it != g_counters.end() && it->second.bytes >= n * sizeof(unsigned);
-}
-
 bool stream_capturing(cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {

@@ -1437,12 +1437,12 @@ bool tc_walk(const GemmProblem &p, const hml_sgemm_config &c, int bn, int k_pad,
 bool tail_buffers(cudaStream_t s, TcWalk *w) {
   const size_t sms = static_cast<size_t>(sm_count());
   const size_t bytes = sms * kTcShapes[kNumTcShapes - 1].bn * kBM * sizeof(float);
-  const bool held = workspace_held(2, bytes, s) && tile_counters_held(sms, s);
+  const bool held = workspace_held(2, bytes, s);  // and with it the counters
   if (held && w->tail == 0) return true;
   if (!held && stream_capturing(s)) return false;
-  void *ws = nullptr;
-  if (workspace_slot(2, bytes, s, &ws) != HML_STATUS_SUCCESS ||
-      tile_counters(sms, s, &w->arrivals) != HML_STATUS_SUCCESS) {
+  void *ws = nullptr;  // (the counters first: slot 2 held means both are)
+  if (tile_counters(sms, s, &w->arrivals) != HML_STATUS_SUCCESS ||
+      workspace_slot(2, bytes, s, &ws) != HML_STATUS_SUCCESS) {
     cudaGetLastError();
     return false;
   }
