@@ -51,6 +51,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -58,6 +59,7 @@
 #include "hml_internal.h"
 #include "hml_lines.h"
 #include "hml_tcgen05.cuh"
+#include "hml_walk.h"
 
 namespace hml {
 namespace {
@@ -319,24 +321,6 @@ struct TcArgs {
 };
 
 // ------------------------------------------------------------ B planes
-// How the threads of a splitting kernel walk B's (n, 8-deep k) chunks:
-// consecutive threads along its contiguous dimension, so that whole sectors
-// are read.  (Along k always, an N-contiguous 4096 x 128 B took 5.3 us, 4.1
-// along n; the B of 56 uneven problems 22 us, now 16.)  32-bit indices: 2^32
-// chunks would be planes of 200 GB.
-struct SplitWalk {
-  bool nfast;
-  unsigned inner, chunks;
-  __device__ SplitWalk(int64_t sbk, int64_t sbn, int n_pad, int k_pad)
-      : nfast(sbn == 1 && sbk != 1), inner(nfast ? n_pad : k_pad / 8),
-        chunks(static_cast<unsigned>(n_pad) * (k_pad / 8)) {}
-  __device__ __forceinline__ void at(unsigned c, int *n, int *k0) const {
-    const unsigned o = c / inner, i = c - o * inner;
-    *n = static_cast<int>(nfast ? i : o);
-    *k0 = static_cast<int>(nfast ? o : i) * 8;
-  }
-};
-
 // planes[p][n][k] (k contiguous, zero padded to n_pad x k_pad): NS BF16
 // planes, or for NS = 4 two 32-bit TF32 planes, hi = TF32(x) and
 // lo = TF32(x - hi).
@@ -346,8 +330,9 @@ __global__ void split_b_kernel(const float *B, int64_t sbk, int64_t sbn, int K, 
   // the tensor-core kernel that reads the planes is launched as a
   // programmatic dependent: its set-up and A loads overlap this kernel
   allow_dependent_launch();
-  const SplitWalk walk(sbk, sbn, n_pad, k_pad);
-  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < walk.chunks;
+  using Index = std::conditional_t<NS <= 2, uint64_t, uint32_t>;
+  const SplitWalk<Index> walk(sbk, sbn, n_pad, k_pad);
+  for (Index c = blockIdx.x * blockDim.x + threadIdx.x; c < walk.chunks;
        c += gridDim.x * blockDim.x) {
     int n, k0;
     walk.at(c, &n, &k0);
@@ -2102,8 +2087,9 @@ template <int NS>
 __global__ void split_b_batch_kernel(const TcSplitDesc *descs) {
   allow_dependent_launch();  // the tensor-core kernels wait for the planes
   const TcSplitDesc d = descs[blockIdx.y];
-  const SplitWalk walk(d.sbk, d.sbn, d.n_pad, d.k_pad);
-  for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < walk.chunks;
+  using Index = std::conditional_t<NS <= 2, uint64_t, uint32_t>;
+  const SplitWalk<Index> walk(d.sbk, d.sbn, d.n_pad, d.k_pad);
+  for (Index c = blockIdx.x * blockDim.x + threadIdx.x; c < walk.chunks;
        c += gridDim.x * blockDim.x) {
     int n, k0;
     walk.at(c, &n, &k0);
