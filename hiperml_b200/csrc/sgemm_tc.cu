@@ -175,11 +175,13 @@ __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi) {
 // lanes' loads to return nor keeps their use from being scheduled behind it,
 // and TMA refills the slot at once (a build with registers to spare did so,
 // and lost rows).  A slot is released after the block's first TMEM store,
-// which takes words of values from all of the row -- except in a ring of 2 or 4
-// slots (EARLY), which cannot wait for the operand stage that store needs
-// (8192^3 with 2 slots 5.95 ms, 6.58 with the later release; 18944 x 64 x 4096
-// with 4 74.8 us, 77.0): there the arriving lane comes from a vote on words w
-// computed from every value.
+// which takes words of values from all of the row -- except (EARLY) in a ring of
+// 2 or 4 slots, which cannot wait for the operand stage that store needs (8192^3
+// with 2 slots 5.95 ms, 6.58 with the later release; 18944 x 64 x 4096 with 4
+// 74.8 us, 77.0), and in 128-wide BF16 tiles at any depth (18944 x 128 x 4096, 8 slots,
+// 100.1 us, 104.2; 20000 x 300 x 6144 518, 540; narrower tiles do better later:
+// 18944 x 16 x 4096 row-major 64.8, 62.2): there the arriving lane comes from a
+// vote on words w computed from every value.
 template <int N>
 __device__ __forceinline__ void release_early(uint64_t *bar, const uint32_t (&w)[N], int lane) {
   uint32_t all = w[0];
@@ -1313,9 +1315,10 @@ hml_status launch_tc_planes(const GemmProblem &p, const hml_sgemm_config &c,
   args.err = err;
   args.bexp = bexp;
   const size_t smem = tc_plan_bytes(BN, NS, plan, AM);
+  constexpr bool kGrid = !PERSIST && !am_unaligned(AM);
   void (*kern)(AMaps<AM>, CUtensorMap, TcArgs) =
-      plan.sa <= 4 ? tc_kernel<BN, NS, AM, PERSIST, !PERSIST && !am_unaligned(AM)>
-                   : tc_kernel<BN, NS, AM, PERSIST, false>;
+      plan.sa <= 4 ? tc_kernel<BN, NS, AM, PERSIST, kGrid>
+                   : tc_kernel<BN, NS, AM, PERSIST, kGrid && BN == 128 && NS <= 3>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e == cudaSuccess && c.split_k > 8)
