@@ -148,6 +148,15 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const void *tmap, ui
       : "memory");
 }
 
+// For a tensor map in device memory, by each CTA before its first load with it:
+// TMA's descriptor cache is not coherent with what wrote the map (a copy by the
+// host, here), and an earlier map at the same address may be in it still.
+__device__ __forceinline__ void acquire_tmap(const void *tmap) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(
+                   reinterpret_cast<uint64_t>(tmap))
+               : "memory");
+}
+
 __device__ __forceinline__ void prefetch_tmap(const void *tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }

@@ -1827,6 +1827,11 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       const unsigned nitems = static_cast<unsigned>(args.nitems);
       const TcBatchItem none = {kNoItem, 0, 0, 0};
       TcBatchItem nxt = q[0] < nitems ? args.items[q[0]] : none;
+      // the next item's map, acquired before it is used or prefetched
+      auto acquire = [&]() {
+        if (nxt.prob != kNoItem) acquire_tmap(args.tmA + nxt.prob);
+      };
+      acquire();
       for (int j = 0;; ++j) {
         const int r = j % kItemRing;
         if (!mbar_wait(&iempty[r], ((j / kItemRing) & 1) ^ 1, args.err, kDevErrEmptyBarrier))
@@ -1865,6 +1870,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
           if (known && kq == 1) {  // (an item has at least two blocks)
             // the next item's record and map, behind the loads just issued
             nxt = q[0] < nitems ? args.items[q[0]] : none;
+            acquire();
             if (nxt.prob != kNoItem) prefetch_tmap(args.tmA + nxt.prob);
           }
         }
@@ -1873,6 +1879,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
           q[0] = atomicAdd(&args.queue[0], 1u);
           w = 1;
           nxt = q[0] < nitems ? args.items[q[0]] : none;
+          acquire();
         }
       }
       // every atomic taken ahead has returned (its register is read) before
@@ -1892,6 +1899,7 @@ __global__ void __launch_bounds__(tcb_warps(BN, NS) * 32, 1) tc_batch_kernel(TcB
       bool ok = cur.fetch(args, ifull, iempty, iring, false, lane);
       for (int blk = 0; ok && !cur.end;) {
         const CUtensorMap *tm = args.tmB + cur.it.prob;
+        if (cur.c == 0) acquire_tmap(tm);
         const int n0 = cur.it.tn * BN;
         const int np = cur.pr->n_pad;
         for (int kb = 0; kb < P; ++kb, ++blk) {
