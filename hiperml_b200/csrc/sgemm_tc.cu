@@ -1651,7 +1651,7 @@ struct TcBatchProblem {
   int n_pad;  // rows of one B plane
 };
 
-struct TcBatchItem {
+struct alignas(16) TcBatchItem {
   int prob, tm, tn;
   int cpt_akc;  // 2 * (64-deep chunks of K) + (A is K-contiguous): the
                 // problem's, beside the tile so that a role that takes the
@@ -1669,6 +1669,7 @@ struct TcBatchArgs {
   unsigned *queue;              // [2]: queue head, CTAs finished (zero between launches)
   int sa, so;
   int first;                    // the plan's first tile kernel
+  int zero;                     // 0 (see settled)
   int *err;
 };
 
@@ -1696,6 +1697,20 @@ __device__ __forceinline__ int queue_ahead(int cpt, unsigned taken, unsigned nit
 // of the sequence is read from ring slot j % kItemRing once published, and
 // the slot is released right after the read (every role reads every item:
 // the roles count chunks across item boundaries).
+//
+// The fields a role keeps are taken through an ALU step right where the record
+// is read (`zero` is 0, which the compiler does not know).  Without it the
+// issuers' code compared an item's chunk count before the load of it had
+// returned where the way from one to the other was the loop's back edge alone
+// -- at an issuer whose turn the item's only chunk was not -- and took the count
+// of the item before: it then waited out its limit for a chunk too many (plans
+// of problems of K <= 256, in one launch of 20; the results were right, 2 s
+// late).
+__device__ __forceinline__ int settled(int v, int zero) {
+  asm volatile("xor.b32 %0, %0, %1;" : "+r"(v) : "r"(zero));
+  return v;
+}
+
 struct QueueCursor {
   TcBatchItem it;
   const TcBatchProblem *pr;
@@ -1709,7 +1724,11 @@ struct QueueCursor {
     bool w = mbar_wait(&ifull[r], (j / kItemRing) & 1, a.err, kDevErrFullBarrier);
     if (warp_role) w = __all_sync(0xffffffffu, w);
     if (!w) return false;
-    it = ring[r];
+    const TcBatchItem rec = ring[r];
+    it.prob = settled(rec.prob, a.zero);
+    it.tm = settled(rec.tm, a.zero);
+    it.tn = settled(rec.tn, a.zero);
+    it.cpt_akc = settled(rec.cpt_akc, a.zero);
     if (warp_role) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&iempty[r]);
