@@ -202,6 +202,28 @@ hml_status select_config(const GemmProblem &p, hml_sgemm_config *c, cudaStream_t
   return HML_STATUS_SUCCESS;
 }
 
+// The BF16X6 tile of a problem with an unaligned A that an addressable one would
+// be SIMT for, or one of K < 256 taken whole: the narrowest whose grid is one wave at most, K split as ever.
+// These are short, and their time is a CTA's rather than the machine's (B200, K
+// odd, row-major, the tile that holds N / this one / SIMT: 1501 x 300 x 101 25.1,
+// 15.5, 15.5 us; 3257 x 104 x 127 24.0, 13.1, 18.9; 1021 x 130 x 301 25.1, 13.1,
+// 17.2; 1501 x 40 x 601 18.9, 14.8, 16.9).  From K = 256 on the measured
+// BF16X6 choice is the better one (1021 x 256 x 601 16.8 us, 25.0).
+static hml_sgemm_config unaligned_tile(const GemmProblem &p) {
+  hml_sgemm_config c = heuristic_config(p, HML_ALGO_BF16X6);
+  const int64_t rows = (static_cast<int64_t>(p.M) + 127) / 128;
+  for (int v = c.variant - 1; v >= 0; --v) {
+    int bm, bn;
+    tc_shape(v, &bm, &bn);
+    const int64_t tiles = rows * ((p.N + bn - 1) / bn);
+    if (tiles > sm_count()) break;
+    c.tile_n = bn;
+    c.variant = v;
+    c.split_k = choose_split(tiles, p.K, 1, 256);
+  }
+  return c;
+}
+
 // Where the tensor cores take a problem whose A TMA cannot address as it
 // stands: wherever they would take it with an addressable A, and where SIMT
 // would from M K max(N, 8) = 2^25 on, with 40 row tiles from M K N = 2^24 on.
@@ -234,7 +256,7 @@ hml_status select_auto(const GemmProblem &p, hml_sgemm_config *c, bool *unaligne
   if (c->algo == HML_ALGO_SIMT &&
       (p.K < 100 || (mk * std::max(p.N, 8) < 0x1p25 && (p.M < 40 * 128 || mk * p.N < 0x1p24))))
     return check_config_ok(p, *c) ? HML_STATUS_SUCCESS : select_config(p, c, s);
-  if (c->algo != HML_ALGO_BF16X6) *c = heuristic_config(q, HML_ALGO_BF16X6);
+  if (c->algo != HML_ALGO_BF16X6 || (p.K < 256 && c->split_k == 1)) *c = unaligned_tile(q);
   *unaligned = true;
   return HML_STATUS_SUCCESS;
 }
