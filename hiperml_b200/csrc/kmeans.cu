@@ -157,10 +157,11 @@ __device__ __forceinline__ void push_close(unsigned *ccount, uint2 *citems, int6
 // among equal ones -- the first minimum in k order, the reference's pick.
 // xs lies on a 16-byte boundary: the warp reads it four elements a load.  The
 // loads bound the settling: 1M x 32 points, k = 64, all of them close calls
-// 1363 us, 1558 one element a load.
+// 1363 us, 1558 one element a load.  Points below 16 dimensions keep that, as the
+// loop over the rest (1M x 7, k = 64 1179 us, 1237 so).
 __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, const float *cs,
                                                     int k, const float *cn, float lim) {
-  const int lane = threadIdx.x & 31, st = d + 1;
+  const int lane = threadIdx.x & 31, st = d + 1, dv = d >= 16 ? d : 0;
   float bd = FLT_MAX;
   int bk = -1;
   for (int c = lane; c < k; c += 32) {
@@ -168,7 +169,7 @@ __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, cons
     if (lim < INFINITY) {
       float dot = 0.0f;
       int j = 0;
-      for (; j + 4 <= d; j += 4) {
+      for (; j + 4 <= dv; j += 4) {
         const float4 v = *reinterpret_cast<const float4 *>(xs + j);
         dot = fmaf(v.x, cp[j], dot);
         dot = fmaf(v.y, cp[j + 1], dot);
@@ -184,7 +185,7 @@ __device__ __forceinline__ uint32_t exact_pick_smem(const float *xs, int d, cons
       dist = __fmaf_rn(delta, delta, dist);
     };
     int j = 0;
-    for (; j + 4 <= d; j += 4) {
+    for (; j + 4 <= dv; j += 4) {
       const float4 v = *reinterpret_cast<const float4 *>(xs + j);
       add(v.x, cp[j]);
       add(v.y, cp[j + 1]);
