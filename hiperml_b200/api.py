@@ -229,7 +229,7 @@ def kmeans_assign(points, centroids, out=None, stream=None, count_exact=False,
     bit), and with ``count_exact`` also the number of points whose candidates
     were resolved with the reference's own arithmetic.  ``method``: 0 = the
     library's choice, 1 = the tiled SIMT form with the argmin fused, 2 = the
-    SGEMM form (products through HBM), 3 = the tensor-core form (BF16X3
+    SGEMM form (products through HBM), 3 = the tensor-core form (FP16X3
     products in TMEM, the argmin read from the accumulator; 4 <= d <= 64 with
     d a multiple of 4, at most 256 centroids)."""
     import torch

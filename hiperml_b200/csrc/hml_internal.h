@@ -73,8 +73,9 @@ hml_status launch_scale(float *C, int M, int N, int64_t scm, int64_t scn, float 
                         cudaStream_t s);
 hml_status launch_simt(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s);
 // waves: a split_k = 1 configuration whose grid would end in a partial wave
-// runs that wave's rows as a second grid split in K (automatic selection
-// only; an explicitly given configuration runs exactly as given).
+// runs that wave's rows split in K, in a persistent grid or a second one, and a
+// ring of 4 slots may run with 6 (automatic selection only; an explicitly given
+// configuration runs exactly as given).
 hml_status launch_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream_t s,
                      bool waves = false);
 // The split-BF16 form (BF16X6) of a problem whose A TMA cannot address as it

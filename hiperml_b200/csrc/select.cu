@@ -156,14 +156,13 @@ bool v1_rule_config(const GemmProblem &p, int K_row, int N_row, hml_sgemm_config
 // that is always the better one; the network, smooth in N and M, misses it
 // near the edges (65536 x 64 x 4096, A K-contiguous: 311 us with the 128-wide
 // tile it takes, 238 with the 64-wide; 14031 x 80 x 1488: 36 us with the
-// 128-wide, 50 with two 64-wide).  Over
-// 5000 measured shapes:
-//   * a tile twice as wide as N needs was at best 1.4 % faster (288 shapes with
-//     32 < N <= 64; at the median 15 % slower; narrower N likewise);
-//   * several narrower tiles were not faster by 3 % in any of 251 shapes whose
-//     row tiles fill more than half of the SMs but one wave, or two waves and
-//     more (at the median 20 to 40 % slower; elsewhere they often win);
-//   * from two waves on, K was better whole in all of 141 shapes.
+// 128-wide, 50 with two 64-wide).  Timed both ways:
+//   * a tile twice as wide as N needs is no faster (32 < N <= 64 15 % slower at
+//     the median, narrower N likewise);
+//   * several narrower tiles are no faster where the row tiles fill more than
+//     half of the SMs but one wave, or two waves and more (20 to 40 % slower at
+//     the median; elsewhere they often win);
+//   * from two waves on, K is better whole.
 // The family stays the network's: the SIMT sums of a short K are closer to the
 // exact ones (about 1e-7 of the largest, BF16X6 5e-7).
 static void fit_tile_to_n(const GemmProblem &p, hml_sgemm_config *c) {

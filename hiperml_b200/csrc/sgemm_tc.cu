@@ -1395,8 +1395,10 @@ hml_status launch_tc_waves(const GemmProblem &p, const hml_sgemm_config &c,
 // one wave on when the split tail occupies half of the SMs (28416 x 32 x 1504
 // 45.3 -> 43.3; a smaller tail's sum through memory costs what is saved:
 // 21001 x 100 x 501 35.4 -> 37.4, 19200 x 128 x 4096 115 -> 112).  Several
-// column tiles at a large K stay with the grids: 8192^3 6.45 ms against 6.70
-// (8192 x 4096 x 2048 825 -> 721 us).
+// column tiles: over eight shapes from 65536 x 256 to 8192 x 8192, both orders of
+// A, the persistent form was 1.1 to 1.3 times as fast at K = 512 (65536 x 256 128
+// -> 97 us), 1.0 to 1.1 at 2048, within 4 % either way at 4096 and beyond, except
+// 8192^3, where the grids are faster (5.38 ms, 5.85).
 bool tc_walk(const GemmProblem &p, const hml_sgemm_config &c, int bn, int k_pad, int n_pad,
              TcWalk *w) {
   const int64_t tiles =

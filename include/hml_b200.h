@@ -106,15 +106,17 @@ const char *hml_version(void);
  * (environment: HML_PREDICTOR=<file> names another, HML_PREDICTOR=none
  * disables it).  When the chosen tensor-core configuration has split_k = 1
  * and its grid of row tiles would end in a wave that leaves at least half of
- * the SMs idle, the rows of that last wave run as a second grid with K split
- * across the idle SMs (those rows then carry split-K rounding, within the
- * same error bounds; hml_sgemm_ex_config runs a configuration exactly as
- * given).  A problem whose A (the operand of the longer dimension) TMA cannot
+ * the SMs idle, the rows of that last wave run with K split across the idle
+ * SMs, in the same persistent grid or a second one (those rows then carry
+ * split-K rounding, within the same error bounds), and a ring of 4 slots may
+ * run with 6 (the same bits); hml_sgemm_ex_config runs a configuration exactly
+ * as given.  A problem whose A (the operand of the longer dimension) TMA cannot
  * address as it stands -- a base or leading dimension that is not a multiple
  * of 16 bytes -- runs as BF16X6 through four strided views of A where that is
  * faster than the SIMT tiles; hml_sgemm_ex_config, which runs configurations
  * as given, refuses the tensor-core ones for such an A, and
- * hml_sgemm_select reports a configuration that it takes.  Replaces the launch half of
+ * hml_sgemm_select reports a configuration that it takes.  A record that the
+ * program tuned or loaded for exactly such a shape stands, if it can read A.  Replaces the launch half of
  * hmlSgemm (src/hml_sgemm.cu:120-211 in the reference), generalised to
  * both storage orders, transposes and leading dimensions. */
 hml_status hml_sgemm_ex(hml_order order, hml_op transA, hml_op transB, int M,
@@ -463,7 +465,7 @@ hml_status hml_kmeans_assign(const float *points, int num_points, int dims,
  * SIMT GEMM with the argmin in its epilogue), 2 = the SGEMM form (the
  * products through HBM, num_points x num_clusters floats of workspace, then a
  * pick kernel; HML_STATUS_NOT_SUPPORTED above 51200 clusters), 3 = the
- * tensor-core form (BF16X3 products on tcgen05 into TMEM, the argmin read
+ * tensor-core form (FP16X3 products on tcgen05 into TMEM, the argmin read
  * from the accumulator; HML_STATUS_NOT_SUPPORTED unless dims is a multiple
  * of 4 in 4..64, points is 16-byte aligned and num_clusters <= 256).  When
  * exact_count (a device counter) is not NULL, the number of points whose
