@@ -492,6 +492,9 @@ hml_status batch_plan_create(hml_order order, const hml_gemm_desc *descs, int co
   if (e == cudaSuccess && !items.empty())
     e = cudaMemcpy(base + oi, items.data(), items.size() * sizeof(BatchItem),
                    cudaMemcpyHostToDevice);
+  // a copy from pageable memory may return before it has arrived, and the plan
+  // may run on a stream that does not wait for the default one
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   if (e != cudaSuccess) {
     note_cuda_error(e, "batch plan upload");
     cudaFree(pl->dev);
