@@ -61,6 +61,14 @@
 #include "hml_tcgen05.cuh"
 #include "hml_walk.h"
 
+// The forms are compiled into a module each, so that a program loads the one it
+// uses: this file alone is BF16X6 with the batches, and sgemm_tc_x3.cu, _tf32.cu
+// and _fp16.cu include it for the others (HML_TC_PART is their NS).  The first
+// call of a process took 28 ms with one module of all, 12 so.
+#ifndef HML_TC_PART
+#define HML_TC_PART 0
+#endif
+
 namespace hml {
 namespace {
 
@@ -292,7 +300,7 @@ __device__ __forceinline__ float maxabs32(const float (&x)[32]) {
 }
 
 // 2^e as a float for e in [-149, 127] (denormal below -126), 0 below.
-__device__ __forceinline__ float exp2_int(int e) {
+[[maybe_unused]] __device__ __forceinline__ float exp2_int(int e) {
   if (e >= -126) return __int_as_float((min(e, 127) + 127) << 23);
   if (e >= -149) return __int_as_float(1 << (e + 149));
   return 0.0f;
@@ -1238,10 +1246,12 @@ __global__ void __launch_bounds__(tc_warps(BN, NS) * 32, 1)
 
 }  // namespace
 
+#if HML_TC_PART == 0
 bool tc_config_fits(int bn, int ns, int stages) {
   TcPlan pl;
   return tc_plan(bn, ns, stages, &pl);
 }
+#endif
 
 namespace {
 
@@ -1542,7 +1552,67 @@ hml_status run_tc_unaligned(const GemmProblem &p, const hml_sgemm_config &c, cud
   return p.a_kcontig() ? run_tc<BN, 3, kAKU>(p, c, s, true) : run_tc<BN, 3, kAMU>(p, c, s, true);
 }
 
+// Where the allocation-free entry point keeps B's planes and its error word.
+struct NoAllocAddrs {
+  void *scratch = nullptr;
+  int *err = nullptr;
+};
+
+// The launch of run_tc with the B planes in the static array and the static
+// error word.
+template <int BN, int NS, int AM>
+hml_status run_tc_static(const GemmProblem &p, const hml_sgemm_config &c, const NoAllocAddrs &a,
+                         cudaStream_t s) {
+  const int k_pad = ((p.K + kChunkK - 1) / kChunkK) * kChunkK;
+  const int n_pad = ((p.N + BN - 1) / BN) * BN;
+  auto *planes = static_cast<__nv_bfloat16 *>(a.scratch);
+  hml_status st = split_b<NS>(p, planes, k_pad, n_pad, s);
+  if (st != HML_STATUS_SUCCESS) return st;
+  return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, a.err, s, false);
+}
+
+template <int NS>
+hml_status run_tc_static_ns(const GemmProblem &p, const hml_sgemm_config &c,
+                            const NoAllocAddrs &a, cudaStream_t s) {
+  const bool ak = p.a_kcontig();
+  switch (c.tile_n) {
+    case 16: return ak ? run_tc_static<16, NS, kAK>(p, c, a, s)
+                       : run_tc_static<16, NS, kAM>(p, c, a, s);
+    case 32: return ak ? run_tc_static<32, NS, kAK>(p, c, a, s)
+                       : run_tc_static<32, NS, kAM>(p, c, a, s);
+    case 64: return ak ? run_tc_static<64, NS, kAK>(p, c, a, s)
+                       : run_tc_static<64, NS, kAM>(p, c, a, s);
+    case 128: return ak ? run_tc_static<128, NS, kAK>(p, c, a, s)
+                        : run_tc_static<128, NS, kAM>(p, c, a, s);
+    default: return HML_STATUS_INVALID_VALUE;
+  }
+}
+
 }  // namespace
+
+#if HML_TC_PART
+#define HML_TC_NAME2(name, part) name##part
+#define HML_TC_NAME(name, part) HML_TC_NAME2(name, part)
+hml_status HML_TC_NAME(run_tc_part, HML_TC_PART)(const GemmProblem &p, const hml_sgemm_config &c,
+                                                 cudaStream_t s, bool waves) {
+  return run_tc_ns<HML_TC_PART>(p, c, s, waves);
+}
+#if HML_TC_PART == 2
+hml_status run_tc_static_part2(const GemmProblem &p, const hml_sgemm_config &c, void *scratch,
+                               int *err, cudaStream_t s) {
+  NoAllocAddrs a;
+  a.scratch = scratch;
+  a.err = err;
+  return run_tc_static_ns<2>(p, c, a, s);
+}
+#endif
+}  // namespace hml
+#else
+hml_status run_tc_part2(const GemmProblem &, const hml_sgemm_config &, cudaStream_t, bool);
+hml_status run_tc_part4(const GemmProblem &, const hml_sgemm_config &, cudaStream_t, bool);
+hml_status run_tc_part5(const GemmProblem &, const hml_sgemm_config &, cudaStream_t, bool);
+hml_status run_tc_static_part2(const GemmProblem &, const hml_sgemm_config &, void *, int *,
+                               cudaStream_t);
 
 int tc_num_shapes() { return kNumTcShapes; }
 void tc_shape(int v, int *bm, int *bn) {
@@ -1589,10 +1659,10 @@ hml_status launch_tc(const GemmProblem &p, const hml_sgemm_config &c, cudaStream
   hml_status st = check_tc(p, c);
   if (st != HML_STATUS_SUCCESS) return st;
   switch (c.algo) {
-    case HML_ALGO_BF16X3: return run_tc_ns<2>(p, c, s, waves);
+    case HML_ALGO_BF16X3: return run_tc_part2(p, c, s, waves);
     case HML_ALGO_BF16X6: return run_tc_ns<3>(p, c, s, waves);
-    case HML_ALGO_FP16X3: return run_tc_ns<5>(p, c, s, waves);
-    default: return run_tc_ns<4>(p, c, s, waves);
+    case HML_ALGO_FP16X3: return run_tc_part5(p, c, s, waves);
+    default: return run_tc_part4(p, c, s, waves);
   }
 }
 
@@ -2438,10 +2508,6 @@ static __device__ int g_noalloc_error;
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
-struct NoAllocAddrs {
-  void *scratch = nullptr;
-  int *err = nullptr;
-};
 NoAllocAddrs g_noalloc_addr[kNoAllocMaxDevices];
 
 // Device addresses of the scratch array and the error word on the current
@@ -2479,36 +2545,6 @@ size_t noalloc_bytes_needed(const GemmProblem &p, const hml_sgemm_config &c) {
   const size_t k_pad = ((static_cast<size_t>(p.K) + kChunkK - 1) / kChunkK) * kChunkK;
   const size_t n_pad = ((static_cast<size_t>(p.N) + c.tile_n - 1) / c.tile_n) * c.tile_n;
   return static_cast<size_t>(ns) * n_pad * k_pad * 2;
-}
-
-// The launch of run_tc with the B planes in the static array and the static
-// error word.
-template <int BN, int NS, int AM>
-hml_status run_tc_static(const GemmProblem &p, const hml_sgemm_config &c, const NoAllocAddrs &a,
-                         cudaStream_t s) {
-  const int k_pad = ((p.K + kChunkK - 1) / kChunkK) * kChunkK;
-  const int n_pad = ((p.N + BN - 1) / BN) * BN;
-  auto *planes = static_cast<__nv_bfloat16 *>(a.scratch);
-  hml_status st = split_b<NS>(p, planes, k_pad, n_pad, s);
-  if (st != HML_STATUS_SUCCESS) return st;
-  return launch_tc_planes<BN, NS, AM>(p, c, planes, k_pad, n_pad, a.err, s, false);
-}
-
-template <int NS>
-hml_status run_tc_static_ns(const GemmProblem &p, const hml_sgemm_config &c,
-                            const NoAllocAddrs &a, cudaStream_t s) {
-  const bool ak = p.a_kcontig();
-  switch (c.tile_n) {
-    case 16: return ak ? run_tc_static<16, NS, kAK>(p, c, a, s)
-                       : run_tc_static<16, NS, kAM>(p, c, a, s);
-    case 32: return ak ? run_tc_static<32, NS, kAK>(p, c, a, s)
-                       : run_tc_static<32, NS, kAM>(p, c, a, s);
-    case 64: return ak ? run_tc_static<64, NS, kAK>(p, c, a, s)
-                       : run_tc_static<64, NS, kAM>(p, c, a, s);
-    case 128: return ak ? run_tc_static<128, NS, kAK>(p, c, a, s)
-                        : run_tc_static<128, NS, kAM>(p, c, a, s);
-    default: return HML_STATUS_INVALID_VALUE;
-  }
 }
 
 }  // namespace
@@ -2566,6 +2602,7 @@ extern "C" hml_status hml_sgemm_ex_config_noalloc(hml_order order, hml_op transA
   NoAllocAddrs addrs;
   st = noalloc_setup(&addrs);
   if (st != HML_STATUS_SUCCESS) return st;
-  return config->algo == HML_ALGO_BF16X3 ? run_tc_static_ns<2>(p, *config, addrs, s)
+  return config->algo == HML_ALGO_BF16X3 ? run_tc_static_part2(p, *config, addrs.scratch, addrs.err, s)
                                          : run_tc_static_ns<3>(p, *config, addrs, s);
 }
+#endif  // HML_TC_PART

@@ -1,0 +1,3 @@
+// The BF16X3 form's kernels (sgemm_tc.cu), a module of their own.
+#define HML_TC_PART 2
+#include "sgemm_tc.cu"
