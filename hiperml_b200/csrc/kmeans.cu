@@ -696,11 +696,11 @@ __global__ void __launch_bounds__(kTThreads, 2) kmeans_resident_kernel(
 // limit): g in packed FP32x2 adds, the smallest by 3-input minima (half an
 // instruction a value), then the sign bits of g - lim shifted into a mask, in
 // which the first smallest is alone unless the point is a close call.
-// Measured on B200 (whole calls): 1M x 32, k = 64 41 us (65 us with TF32X3
+// Measured on B200 (whole calls): 1M x 32, k = 64 43 us (65 us with TF32X3
 // products, the per-value argmin and separate prep and settle kernels; 21 us
-// of HBM time), k = 256 109 us (162); 1M x 128, k = 64 90 us (709 us on the
-// tiled form; 84 us of HBM time), 1M x 256, k = 64 171 us (1560; 167); 1M x
-// 11, k = 192 85 us (300).  Wide points are bound by HBM, narrow ones by the
+// of HBM time), k = 256 106 us (162); 1M x 128, k = 64 87 us (709 us on the
+// tiled form; 84 us of HBM time), 1M x 256, k = 64 163 us (1560; 167); 1M x
+// 11, k = 192 94 us (300).  Wide points are bound by HBM, narrow ones by the
 // groups' own instructions and the latencies between them.
 constexpr int kTcMaxK = 256;                     // centroids (padded to 16)
 constexpr int kTcMaxPlanes = 128 * 1024;         // bytes of the centroids' planes
